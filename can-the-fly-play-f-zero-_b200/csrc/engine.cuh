@@ -12,9 +12,10 @@
 //   delay line  acc[S][B][n_pad] (i32 or i64): synaptic input of the next S ticks (slot = tick mod
 //               S, S = 2 x the persistent engine's epoch, at least 2), rows padded to 16 entries so
 //               that every row starts on a 64-byte boundary (TMA bulk copies);
-//               items[R][n_groups][n_seg][cap_c] int2: spike work lists of the last R = n_delay+1
-//               steps, one per instance group and segment (the pairs one persistent CTA owns);
-//               item_count[R][n_groups][n_seg]; pring[R_pl][B][n_ppost] i64: plastic input (R_pl = n_delay + epoch: a slot
+//               items[R][n_groups][cap_c] int2: spike work lists of the last R = n_delay + K steps (K: the
+//               persistent engine's epoch, 1 without it; a list is emptied K steps before it is filled
+//               again), one per instance group; item_count[R][n_groups];
+//               pring[R_pl][B][n_ppost] i64: plastic input (R_pl = n_delay + K: a slot
 //               is cleared by its reader at least one epoch before anyone pushes into it again);
 //               with pull propagation also masks[R][n][ceil(B/64)] u64: which instances each
 //               neuron spiked in, and the connectome by postsynaptic neuron (colptr, cpre, ccnt/cwfx)
@@ -63,13 +64,11 @@ struct DevState {
     void* acc;                 // [n_slots][B][n_pad]
     int32_t n_slots;
     int64_t* pring;
-    int2* items;               // [R][n_groups][n_seg][cap_c]
-    int32_t* item_count;       // [R][n_groups][n_seg]
-    int64_t cap_c;             // items per (step, group, segment) list
+    int2* items;               // [R][n_groups][cap_c]
+    int32_t* item_count;       // [R][n_groups]
+    int64_t cap_c;             // items per (step, group) list
     int32_t group;             // instances per group (group of instance b = b / group)
     int32_t n_groups;
-    int32_t n_seg;             // segments per group: the CTAs of the persistent plan (1 without one)
-    int64_t seg_pairs;         // pairs per segment; pair (b, i) = (b mod group) * n_pad + i
     const int64_t* reset_tick;
     const int64_t* stop_tick;
     unsigned long long* masks; // pull propagation: [R][n][mask_words] spiking instances per neuron (or nullptr)
@@ -107,20 +106,13 @@ template <typename Real> __device__ __forceinline__ const Lif<Real>& lif_of(cons
 template <> __device__ __forceinline__ const Lif<float>& lif_of<float>(const DevNet& N) { return N.L32; }
 template <> __device__ __forceinline__ const Lif<double>& lif_of<double>(const DevNet& N) { return N.L64; }
 
-__device__ __forceinline__ int2* list_of(const DevState& S, int64_t slot, int32_t q, int32_t c)
+__device__ __forceinline__ int2* list_of(const DevState& S, int64_t slot, int32_t q)
 {
-    return S.items + (((int64_t)slot * S.n_groups + q) * S.n_seg + c) * S.cap_c;
+    return S.items + ((int64_t)slot * S.n_groups + q) * S.cap_c;
 }
-__device__ __forceinline__ int32_t* count_of(const DevState& S, int64_t slot, int32_t q, int32_t c)
+__device__ __forceinline__ int32_t* count_of(const DevState& S, int64_t slot, int32_t q)
 {
-    return S.item_count + ((int64_t)slot * S.n_groups + q) * S.n_seg + c;
-}
-// list key (group * n_seg + segment) of the pair (b, i)
-__device__ __forceinline__ int32_t list_key(const DevState& S, int64_t n_pad, int32_t b, int32_t i)
-{
-    const int32_t q = b / S.group;
-    const int64_t p = (int64_t)(b - q * S.group) * n_pad + i;
-    return q * S.n_seg + (int32_t)(p / S.seg_pairs);
+    return S.item_count + (int64_t)slot * S.n_groups + q;
 }
 
 // Fire-and-forget reductions into global memory (no value comes back; the address is converted to
@@ -146,7 +138,7 @@ __device__ __forceinline__ int2 make_item(const DevNet& N, int32_t i, int32_t b,
 }
 
 // Append `nch` work items (this lane's spike: chunks 0..nch-1 of row i of instance b) to the list of
-// the lane's (group, segment); one atomic per warp and list (the ballot/shuffle compaction).
+// the lane's group; one atomic per warp and list (the ballot/shuffle compaction).
 __device__ __forceinline__ void warp_append(const DevNet& N, const DevState& S, int64_t slot, int nch, int32_t i,
                                             int32_t b)
 {
@@ -154,7 +146,7 @@ __device__ __forceinline__ void warp_append(const DevNet& N, const DevState& S, 
     const int lane = threadIdx.x & 31;
     unsigned todo = __ballot_sync(FULL, nch > 0);
     if (!todo) return;
-    const int32_t key = nch > 0 ? list_key(S, N.n_pad, b, i) : -1;
+    const int32_t key = nch > 0 ? b / S.group : -1;
     while (todo) {
         const int leader = __ffs(todo) - 1;
         const int32_t kk = __shfl_sync(FULL, key, leader);
@@ -166,12 +158,11 @@ __device__ __forceinline__ void warp_append(const DevNet& N, const DevState& S, 
             if (lane >= o) incl += y;
         }
         const int total = __shfl_sync(FULL, incl, 31);
-        const int32_t q = kk / S.n_seg, c = kk - q * S.n_seg;
         int base = 0;
-        if (lane == 31) base = atomicAdd(count_of(S, slot, q, c), total);
+        if (lane == 31) base = atomicAdd(count_of(S, slot, kk), total);
         base = __shfl_sync(FULL, base, 31);
         if (mine) {
-            int2* list = list_of(S, slot, q, c);
+            int2* list = list_of(S, slot, kk);
             const int64_t start = (int64_t)base + incl - nch;
             for (int ch = 0; ch < nch; ch++) {
                 const int64_t p = start + ch;
@@ -261,8 +252,7 @@ __global__ void __launch_bounds__(256) k_update(const DevNet N, const DevState S
     const Lif<Real>& L = lif_of<Real>(N);
     const int64_t t = A.t;
     if (blockIdx.x == 0)       // the lists consumed by the push at t-1 start empty again
-        for (int32_t k = threadIdx.x; k < S.n_groups * S.n_seg; k += blockDim.x)
-            S.item_count[pos_mod(t - N.n_delay, N.R) * S.n_groups * S.n_seg + k] = 0;
+        for (int32_t k = threadIdx.x; k < S.n_groups; k += blockDim.x) *count_of(S, pos_mod(t - N.n_delay, N.R), k) = 0;
     AccT* acc = acc_slot<AccT>(N, S, t);
     Real* V = reinterpret_cast<Real*>(S.v);
     Real* G = reinterpret_cast<Real*>(S.g);
@@ -371,70 +361,25 @@ __device__ __forceinline__ void push_item(const DevNet& N, AccT* acc_b, int64_t 
     }
 }
 
-// Inclusive prefix over the n_seg segment counts of list (slot, q) into `pre` (shared memory),
-// computed by one warp (n_seg <= MAX_SEG); returns the total. Counts are clamped to the capacity.
-constexpr int MAX_SEG = 256;
-__device__ __forceinline__ int32_t segment_prefix(const DevState& S, int64_t slot, int32_t q, int32_t* pre)
+// Items of list (slot, q): its count, clamped to the capacity (L2: other SMs appended to it)
+__device__ __forceinline__ int32_t list_length(const DevState& S, int64_t slot, int32_t q)
 {
-    constexpr int PER_LANE = MAX_SEG / 32;
-    const int lane = threadIdx.x & 31;
-    const int32_t* cnt = count_of(S, slot, q, 0);
-    const int32_t c0 = lane * PER_LANE;
-    int32_t x[PER_LANE];
-#pragma unroll
-    for (int j = 0; j < PER_LANE; j++) x[j] = c0 + j < S.n_seg ? __ldcg(cnt + c0 + j) : 0;   // all in flight
-    int32_t sum = 0;
-#pragma unroll
-    for (int j = 0; j < PER_LANE; j++) {
-        x[j] = (int32_t)min((int64_t)max(x[j], 0), S.cap_c);
-        sum += x[j];
-    }
-    int32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    int32_t run = incl - sum;
-#pragma unroll
-    for (int j = 0; j < PER_LANE; j++) {
-        run += x[j];
-        if (c0 + j < S.n_seg) pre[c0 + j] = run;
-    }
-    return __shfl_sync(0xffffffffu, incl, 31);
+    return (int32_t)min((int64_t)max(__ldcg(count_of(S, slot, q)), 0), S.cap_c);
 }
 
-// Scatter the items [g0, g1) of list (slot of spike step s = t+1-n_delay, group q) into acc_next.
-// The list is the concatenation of its segments, described by their inclusive prefix `pre`; lane
+// Scatter the items [g0, g1) of list (slot of spike step s = t+1-n_delay, group q) into acc_next; lane
 // group `lg` of `n_lg` (LANES lanes each, lane `lane` within it) takes items g0+lg, g0+lg+n_lg, ...
-// and follows the segment boundaries forward (a search only when it crosses one). Items of
-// instance b are skipped unless reset_tick[b - b_base] <= s and t+1 < stop_tick[b - b_base].
+// Items of instance b are skipped unless reset_tick[b] <= s and t+1 < stop_tick[b].
 template <typename AccT, int LANES>
 __device__ __forceinline__ void push_range(const DevNet& N, const DevState& S, int64_t t, int32_t q, AccT* acc_next,
-                                           const int32_t* pre, int64_t g0, int64_t g1, int64_t lg, int64_t n_lg,
-                                           int lane, const int64_t* reset_tick, const int64_t* stop_tick,
-                                           int32_t b_base)
+                                           int64_t g0, int64_t g1, int64_t lg, int64_t n_lg, int lane)
 {
     const int64_t s = t + 1 - N.n_delay;
-    if (s < 0) return;
-    const int64_t slot = pos_mod(s, N.R);
-    int32_t seg = -1;
-    int64_t seg_lo = 0, seg_hi = 0;
+    const int2* list = list_of(S, pos_mod(s, N.R), q);
     for (int64_t g = g0 + lg; g < g1; g += n_lg) {
-        if (g >= seg_hi) {                        // first segment whose prefix exceeds g
-            int32_t lo = seg + 1, hi = S.n_seg - 1;
-            while (lo < hi) {
-                const int32_t mid = (lo + hi) >> 1;
-                if (pre[mid] > g) hi = mid;
-                else lo = mid + 1;
-            }
-            seg = lo;
-            seg_lo = lo > 0 ? pre[lo - 1] : 0;
-            seg_hi = pre[lo];
-        }
-        const int2 item = __ldcg(list_of(S, slot, q, seg) + (g - seg_lo));
+        const int2 item = __ldcg(list + g);
         const int32_t b = item.y >> CHUNK_BITS;
-        if (s < reset_tick[b - b_base] || t + 1 >= stop_tick[b - b_base]) continue;
+        if (s < S.reset_tick[b] || t + 1 >= S.stop_tick[b]) continue;
         push_item<AccT, LANES>(N, acc_next + (int64_t)b * N.n_pad, (int64_t)(uint32_t)item.x,
                                item.y & ((1 << CHUNK_BITS) - 1), lane);
     }
@@ -460,22 +405,17 @@ __device__ __forceinline__ void clear_mask_slot(const DevNet& N, const DevState&
 template <typename AccT, int LANES>
 __global__ void __launch_bounds__(256) k_push(const DevNet N, const DevState S, int64_t t, int do_push)
 {
-    __shared__ int32_t pre[MAX_SEG];
-    __shared__ int32_t s_total;
     clear_mask_slot(N, S, t);
     if (!do_push || t + 1 - N.n_delay < 0) return;
     AccT* acc = acc_slot<AccT>(N, S, t + 1);
     const int64_t slot = pos_mod(t + 1 - N.n_delay, N.R);
+    __shared__ int32_t s_total;
     for (int32_t q = 0; q < S.n_groups; q++) {
-        if (threadIdx.x < 32) {
-            const int32_t tot = segment_prefix(S, slot, q, pre);
-            if (threadIdx.x == 0) s_total = tot;
-        }
+        if (threadIdx.x == 0) s_total = list_length(S, slot, q);     // (one load per block: they all hit one address)
         __syncthreads();
         const int64_t total = s_total;
         const int64_t g0 = total * blockIdx.x / gridDim.x, g1 = total * (blockIdx.x + 1) / gridDim.x;
-        push_range<AccT, LANES>(N, S, t, q, acc, pre, g0, g1, threadIdx.x / LANES, blockDim.x / LANES,
-                                threadIdx.x % LANES, S.reset_tick, S.stop_tick, 0);
+        push_range<AccT, LANES>(N, S, t, q, acc, g0, g1, threadIdx.x / LANES, blockDim.x / LANES, threadIdx.x % LANES);
         __syncthreads();
     }
 }

@@ -129,7 +129,6 @@ struct fb_brain {
     int32_t max_chunks = 0;
     // plastic
     int64_t n_pl = 0;
-    int32_t pl_mode = 0;              // 0 no plastic synapses, 1 plastic, 2 plastic in long rows
     int32_t n_ppost = 0;
     int64_t* pl_rowptr = nullptr;
     int32_t* pl_pidx = nullptr;
@@ -170,13 +169,11 @@ struct fb_brain {
     int64_t* pring = nullptr;
     int2* items = nullptr;
     int32_t* item_count = nullptr;
-    int64_t cap_c = 0;            // items per (step, group, segment) list (<= cap_alloc)
+    int64_t cap_c = 0;            // items per (step, group) list (<= cap_alloc)
     int64_t cap_alloc = 0;        // ... as allocated
     long long barrier_cycles = BARRIER_TIMEOUT_CYCLES;   // persistent engine's grid-barrier wait budget
     int32_t list_group = 1;       // instances per group (the persistent group size, or B)
     int32_t n_groups = 1;
-    int32_t n_seg = 1;            // segments per group (the persistent CTAs, or 1)
-    int64_t seg_pairs = 0;        // pairs per segment
     unsigned int* bar = nullptr;  // persistent grid-barrier counter
     int32_t* abort_flag = nullptr;
     int2* ext_tab = nullptr;      // persistent engine: input pairs of each CTA
@@ -224,7 +221,7 @@ struct fb_brain {
         S.v = v; S.g = g; S.ref = ref; S.pw = pw; S.ext_idx = ext_idx; S.n_ext = (int32_t)n_ext;
         S.p_ext = p_ext; S.bias_ext = bias_ext; S.acc = acc; S.n_slots = n_slots; S.pring = pring;
         S.items = items; S.item_count = item_count; S.cap_c = cap_c; S.group = list_group;
-        S.n_groups = n_groups; S.n_seg = n_seg; S.seg_pairs = seg_pairs; S.reset_tick = reset_tick;
+        S.n_groups = n_groups; S.reset_tick = reset_tick;
         S.stop_tick = stop_tick; S.err = err_d; S.seed = seed;
         S.masks = masks; S.mask_words = mask_words;
         return S;
@@ -293,12 +290,6 @@ int install_plastic(fb_brain* h, const std::vector<int64_t>& pos)
     if ((rc = upload(&h->pring, ring, tb))) return rc;
     h->n_pl = P.n_pl;
     h->n_ppost = P.n_ppost;
-    {   // long plastic rows (on average two or more plastic synapses per presynaptic neuron with any):
-        // the persistent engine batches their pushes
-        int64_t rows = 0;
-        for (size_t r = 0; r + 1 < P.plr.size(); r++) rows += P.plr[r + 1] > P.plr[r];
-        h->pl_mode = P.n_pl == 0 ? 0 : (P.n_pl >= 2 * std::max<int64_t>(rows, 1) ? 2 : 1);
-    }
     h->plastic = std::move(P);
     return FB_OK;
 }
@@ -387,7 +378,6 @@ extern "C" int fb_create(const fb_params* P, const int64_t* indptr, const int32_
     h->f64 = (flags & FB_FLAG_F64) ? 1 : 0;
     h->n_delay = (int32_t)std::max<int64_t>(1, py_round(P->delay / P->dt));
     h->n_ref = (int32_t)py_round(P->t_ref / P->dt);
-    h->R = h->n_delay + 1;
     h->n_pad = (n + 15) / 16 * 16;
     if (h->n_ref < 0 || h->n_ref > 127) { delete h; return fail(FB_ERR_ARG, "n_ref=%d must fit int8", h->n_ref); }
     int dev_sms = 0;
@@ -428,26 +418,23 @@ extern "C" int fb_create(const fb_params* P, const int64_t* indptr, const int32_
     TRY(dalloc(&h->bar, 1, tb));
     TRY(dalloc(&h->abort_flag, 1, tb));
     int dev_sms2 = h->sm_count;
-    h->plan = plan_persistent(h->n, h->n_pad, h->B, h->f64 != 0, h->n_ref, h->n_delay, (int)ab, dev_sms2, h->device);
-    // the persistent engine runs epochs of K steps between grid barriers: the spikes of an epoch
-    // arrive two epochs later at the earliest when 2K + 1 <= n_delay; 2K accumulator slots
-    h->epoch = h->plan.group > 0 ? std::max(1, std::min(MAX_EPOCH, (h->n_delay - 1) / 2)) : 1;
+    h->plan = plan_persistent(h->n, h->n_pad, h->B, h->f64 != 0, h->n_ref, h->n_delay, dev_sms2, h->device);
+    // the persistent engine runs epochs of K steps between grid barriers: the spikes of an epoch, listed
+    // in the next one, arrive three epochs later at the earliest when 3K <= n_delay; 2K accumulator slots
+    h->epoch = h->plan.group > 0 ? persistent_epoch(h->plan, h->n_pad, h->n_delay, (int)ab) : 1;
     h->n_slots = 2 * h->epoch;
-    h->R_pl = h->n_delay + h->epoch;
+    h->R_pl = h->R = h->n_delay + h->epoch;
     TRY(dalloc((char**)&h->acc, nbp * ab * h->n_slots, tb));
     CU(cudaMemset(h->acc, 0, nbp * ab * h->n_slots));
     h->list_group = h->plan.group > 0 ? h->plan.group : h->B;
     h->n_groups = (h->B + h->list_group - 1) / h->list_group;
     TRY(install_plastic(h, pos));
     TRY(build_ext_table(h));
-    // one list segment per persistent CTA (the pairs it owns); capacity for the worst case, every
-    // pair of the segment firing in the same step
-    h->n_seg = h->plan.group > 0 ? h->plan.ctas : 1;
-    h->seg_pairs = h->plan.group > 0 ? h->plan.per : (int64_t)h->list_group * h->n_pad;
-    h->cap_c = segment_capacity(H, h->n_pad, h->list_group, h->seg_pairs, h->n_seg);
+    // one list per instance group and step; capacity for the worst case, every pair firing in the same step
+    h->cap_c = segment_capacity(H, h->n_pad, h->list_group, (int64_t)h->list_group * h->n_pad, 1);
     h->cap_alloc = h->cap_c;
-    TRY(dalloc(&h->items, (size_t)h->R * h->n_groups * h->n_seg * h->cap_c, tb));
-    TRY(dalloc(&h->item_count, (size_t)h->R * h->n_groups * h->n_seg, tb));
+    TRY(dalloc(&h->items, (size_t)h->R * h->n_groups * h->cap_c, tb));
+    TRY(dalloc(&h->item_count, (size_t)h->R * h->n_groups, tb));
     TRY(dalloc(&h->reset_tick, (size_t)batch, tb));
     TRY(dalloc(&h->stop_tick, (size_t)batch, tb));
     TRY(dalloc(&h->fly_mask, (size_t)batch, tb));
@@ -593,7 +580,7 @@ extern "C" int fb_reset(fb_brain* h, const int32_t* flies, int32_t n_flies, void
             h->mask_from = 0;
             h->masks_dirty = false;
         }
-        CU(cudaMemsetAsync(h->item_count, 0, (size_t)h->R * h->n_groups * h->n_seg * sizeof(int32_t), st));
+        CU(cudaMemsetAsync(h->item_count, 0, (size_t)h->R * h->n_groups * sizeof(int32_t), st));
     }
     k_set_ticks<<<(h->B + 255) / 256, 256, 0, st>>>(h->reset_tick, mask, h->B, h->t);
     CU(cudaGetLastError());
@@ -950,8 +937,8 @@ extern "C" int fb_run(fb_brain* h, int32_t steps, int32_t* counts_out, const uin
         P.epoch = h->epoch;
         P.barrier_cycles = h->barrier_cycles;
         CU(cudaMemsetAsync(h->abort_flag, 0, sizeof(int32_t), st));
-        int rc = launch_persistent(h->plan, h->net(), h->state(), P, h->acc_mode, h->n_pl > 0 ? h->pl_mode : 0,
-                                   kicks != nullptr, record, h->lanes, st);
+        int rc = launch_persistent(h->plan, h->net(), h->state(), P, h->acc_mode, h->n_pl > 0, kicks != nullptr, record,
+                                   st);
         if (rc) return fail(FB_ERR_CUDA, "persistent launch: %s", cudaGetErrorString((cudaError_t)rc));
         h->launches += h->plan.launches_per_run;
         h->pushed_until = std::max<int64_t>(h->pushed_until, h->t + steps + 1);

@@ -20,10 +20,9 @@ import scipy.sparse as sp
 from . import _lib
 from .brain import LIFParams
 
-# Phase stamps of the persistent engine's trace (csrc/persist.cuh): 0 step start, 4 the next step's
-# kicks drawn, 1 slice wait begins, 2 slice in shared memory, 3 neurons advanced, 8 listing warps
-# done; at an epoch's first step 7 / 10 push warps start / done; at its last 5 / 6 grid-barrier
-# arrival / exit.
+# Phase stamps of the persistent engine's trace (csrc/persist.cuh): 0 (and 4, 1, 2) a step's even share of
+# its epoch begins, 3 it ends, 8 listing warps done; at an epoch's first step 7 / 10 push warps start
+# / done; at its last 5 / 9 / 6 grid-barrier arrival / next epoch's kicks drawn / barrier exit.
 TRACE_SLOTS = 11
 
 

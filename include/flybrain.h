@@ -68,7 +68,7 @@ typedef struct {
     int64_t t;            /* simulated steps since the last full reset (BatchBrain.t) */
     uint32_t step_no;     /* global step counter feeding the Poisson hash (BatchBrain.step_no) */
     int64_t launches;     /* kernels launched by this engine so far */
-    int64_t item_capacity;/* spike work items per (step, instance group, list segment) list */
+    int64_t item_capacity;/* spike work items per (step, instance group) list */
     int64_t bytes_device; /* device memory held by the engine */
     double decay_syn;     /* exp(-dt / tau_syn), computed in FP64 on the device */
     double decay_m;       /* dt / tau_m */
@@ -236,11 +236,11 @@ int fb_set_schedule(fb_brain* brain, int32_t engine, int32_t propagation, int32_
 
 /* Phase trace of the persistent engine (diagnostics). `trace` [device] holds `capacity` int64;
  * every later fb_run whose steps * ctas * 11 fits records, per step and CTA, the SM clock at
- * these points, in step order: 0 step start (accumulator slice requested), 4 next step's kicks
- * drawn, 1 waiting for the slice, 2 slice staged, 3 neurons advanced; 8 listing warps done; per
- * epoch of steps between grid barriers, at its first step 7 push warps start and 10 push warps
- * done, at its last step 5 grid-barrier arrival and 6 grid-barrier exit. NULL: off. No
- * counterpart in the reference. */
+ * these points, in step order: 0 step start, 4, 1 and 2 the same, 3 neurons advanced (the steps of
+ * an epoch between grid barriers run together: its span is divided evenly between them); 8 listing
+ * warps done; per epoch, at its first step 7 push warps start and 10 push warps done, at its last
+ * step 5 grid-barrier arrival, 9 the next epoch's kicks drawn and 6 grid-barrier exit (5, 9 and 6 not
+ * for the run's last epoch, which needs no barrier). NULL: off. No counterpart in the reference. */
 int fb_set_trace(fb_brain* brain, long long* trace, int64_t capacity);
 
 /* Limits for fault drills (diagnostics; no counterpart in the reference, whose only guard is a
