@@ -673,9 +673,9 @@ extern "C" int fb_trace_rates(const fb_brain* h, const int32_t* counts, const in
         n_upost < 0)
         return fail(FB_ERR_ARG, "bad arguments");
     CU(cudaSetDevice(h->device));
-    const int64_t work = (int64_t)h->B * (n_upre + n_upost);
+    const int64_t work = (int64_t)n_upre + n_upost;
     if (work == 0) return FB_OK;
-    const int blocks = (int)std::min<int64_t>((work + 255) / 256, (int64_t)h->sm_count * 8);
+    const dim3 blocks((unsigned)((work + 255) / 256), (unsigned)std::min((h->B + TRACE_ROWS - 1) / TRACE_ROWS, 65535));
     k_trace_rates<<<blocks, 256, 0, (cudaStream_t)stream>>>(counts, h->n, h->B, upre, n_upre, trace, a_pre, scale_pre,
                                                             upost, n_upost, rate, a_rate, hz);
     CU(cudaGetLastError());
@@ -694,8 +694,8 @@ extern "C" int fb_delta_apply(fb_brain* h, const int32_t* sel, const int32_t* pr
     CU(cudaSetDevice(h->device));
     DeltaArgs a{h->B, n_flies, n_sel, n_tr, n_x, h->n_pl, sel, pre_k, post_x, trace, x, coef, fly_ptr, fly_slots, sign,
                 wmax, h->pw};
-    const int64_t work = (int64_t)n_sel * n_flies;
-    k_delta_apply<<<(unsigned)((work + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a);
+    const unsigned rows = (unsigned)std::min((n_flies + DELTA_FLIES - 1) / DELTA_FLIES, 65535);
+    k_delta_apply<<<dim3(((unsigned)n_sel + 255u) / 256u, rows), 256, 0, (cudaStream_t)stream>>>(a);
     CU(cudaGetLastError());
     return FB_OK;
 }
@@ -707,8 +707,7 @@ extern "C" int fb_backprop(const fb_brain* h, const int32_t* sel, const int32_t*
     if (n_sel == 0) return FB_OK;
     if (!sel || !pre_l || !post_x || !x || !delta) return fail(FB_ERR_ARG, "NULL argument");
     CU(cudaSetDevice(h->device));
-    const int64_t work = (int64_t)h->B * n_sel;
-    const int blocks = (int)std::min<int64_t>((work + 255) / 256, (int64_t)h->sm_count * 8);
+    const dim3 blocks(((unsigned)n_sel + 255u) / 256u, (unsigned)std::min(h->B, 65535));
     k_backprop<<<blocks, 256, 0, (cudaStream_t)stream>>>(h->B, n_sel, sel, pre_l, post_x, x, n_x, h->pw, h->n_pl,
                                                          (float)h->params.w_syn, delta, n_delta);
     CU(cudaGetLastError());

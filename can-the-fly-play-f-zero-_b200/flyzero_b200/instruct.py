@@ -129,6 +129,10 @@ class BatchInstruct:
         self.rate = torch.zeros((B, len(self.upost)), dtype=torch.float32, device=dev)
         self.upost_group = torch.as_tensor(group_of[self.upost].astype(np.int64), device=dev)
         self.group_members = [np.flatnonzero(group_of[self.upost] == k) for k in range(len(self.names))]
+        # the DN columns of `rate`, group after group: only these are compared with targets and read back
+        cols = np.concatenate(self.group_members)
+        self._dn_cols = torch.as_tensor(cols, device=dev)
+        self._dn_col_group = torch.as_tensor(group_of[self.upost[cols]].astype(np.int64), device=dev)
         self.dn_sel_h = np.flatnonzero(self.mask_h)                      # synapses onto the DNs
         self.dn_sel, self.dn_pre_k, self.dn_post_k = (i32(self.dn_sel_h), i32(self.pre_k_h[self.dn_sel_h]),
                                                       i32(self.post_k_h[self.dn_sel_h]))
@@ -202,11 +206,12 @@ class BatchInstruct:
             new = torch.clamp(self.ib + step, -self.bias_limit, self.bias_limit)
             self.brain.bias_ext[:, self.dn_slots] += new - self.ib
             self.ib = new
-        rate = self.rate.cpu().numpy()
-        out = np.zeros(self.B)
+        rate = self.rate.index_select(1, self._dn_cols).cpu().numpy()
+        out, at = np.zeros(self.B), 0
         for k, mem in enumerate(self.group_members):
             if len(mem):
-                out += np.abs(np.asarray(targets)[:, k] - rate[:, mem].mean(1))
+                out += np.abs(np.asarray(targets)[:, k] - rate[:, np.arange(at, at + len(mem))].mean(1))
+            at += len(mem)
         return np.where(learn, out / len(self.names), 0.0)
 
     def state(self, fly: int) -> dict:
@@ -242,10 +247,8 @@ class BatchInstruct:
 
     def _dn_error(self, tgt):
         """err[b][k] = target of the group of upost_k - rate[b][k] (0 for non-DN targets)."""
-        torch = self._torch()
-        g = self.upost_group
-        e = tgt[:, torch.clamp(g, min=0)] - self.rate
-        self._err.copy_(torch.where(g[None, :] >= 0, e, torch.zeros_like(e)))
+        self._err.index_copy_(1, self._dn_cols, tgt.index_select(1, self._dn_col_group) -
+                              self.rate.index_select(1, self._dn_cols))
         return self._err
 
     def _learn(self, tgt, learn, eta):
