@@ -221,61 +221,62 @@ __global__ void k_eye_delay(const EyeArgs a)
     if (p % (2 * cells) == 0) a.restart[p / (2 * cells)] = 0;
 }
 
-// ---- the whole eye of one instance in one block ----------------------------------------------------
-// The same operations as the four kernels above, in one launch: block b reads its frame once, keeps
-// the grid (luminance, ON/OFF signals, delay arms, colour grids, integral image, float64 contrast)
-// in shared memory, writes its eye neurons' probabilities, then its new delay arms.
+// ---- the same eye in two launches (the default) ----------------------------------------------------------
+// The grid of every instance by one thread per cell, then the neurons of an instance by several blocks.
+// One block per instance (its grid in shared memory) kept 64 instances on 64 of the 148 SMs and waited
+// through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16.5.
 
-struct EyeSmem {
-    int32_t cells, ii, chrom, sust;
-    static constexpr int32_t TAB = 766 + 256;  // pixel luminance by R+G+B, channel quotient by byte
-    __host__ __device__ size_t bytes() const
-    {
-        return (size_t)cells * 8 * sust + (size_t)cells * 4 * (5 + 2 * chrom) + (size_t)ii * 4 * sust + TAB * 4;
-    }
-};
+// x / 3 and x / 255 rounded to nearest for the values a pixel can take (R + G + B and its third, a byte): one
+// Newton correction of the quotient by its exact remainder (Markstein 1990). Checked against the
+// division for all 766 sums and 256 bytes. Tables of the quotients in shared memory cost 3.5 bank cycles a
+// lookup: 9.1 us per 64 frames of 224 x 256 against 7.4.
+__device__ __forceinline__ float eye_quotient(float x, float d, float r)
+{
+    const float q = __fmul_rn(x, r);
+    return __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+}
+__device__ __forceinline__ float eye_lum(float sum) { return eye_quotient(eye_quotient(sum, 3.0f, 1.0f / 3.0f), 255.0f, 1.0f / 255.0f); }
+__device__ __forceinline__ float eye_channel(float byte) { return eye_quotient(byte, 255.0f, 1.0f / 255.0f); }
 
-// A pixel's luminance mean(R, G, B) / 255 depends only on the integer R + G + B (the float sum of
-// three bytes is exact), and a channel value / 255 only on its byte: the tables hold those
-// quotients, computed with the same correctly rounded divisions, so the per-pixel work is a lookup.
+// The sums of one cell: luminance, blue, green (the colours when `chrom`).
 // VEC4: cell 4 and W a multiple of 4, so a cell row is three aligned 32-bit words.
 template <bool VEC4>
-__device__ __forceinline__ void cell_sums(const EyeArgs& a, const uint8_t* fr, bool fl, int32_t y, int32_t x,
-                                          const float* t_lum, const float* t_ch, bool chrom, float& s, float& sb,
-                                          float& sg)
+__device__ __forceinline__ void cell_sums(const EyeArgs& a, const uint8_t* fr, bool fl, int32_t y, int32_t x, bool chrom,
+                                          float& s, float& sb, float& sg)
 {
     s = sb = sg = 0.0f;
     if constexpr (VEC4) {
         const int32_t c0 = fl ? a.W - 4 - 4 * x : 4 * x;
+        uint32_t w[4][3];
 #pragma unroll
         for (int32_t yy = 0; yy < 4; yy++) {
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(fr + ((int64_t)(4 * y + yy) * a.W + c0) * 3);
-            const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2);
-            uint32_t ch[12];
+            const uint32_t* p = reinterpret_cast<const uint32_t*>(fr + ((int64_t)(4 * y + yy) * a.W + c0) * 3);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                ch[j] = (w0 >> (8 * j)) & 255u;
-                ch[4 + j] = (w1 >> (8 * j)) & 255u;
-                ch[8 + j] = (w2 >> (8 * j)) & 255u;
+            for (int j = 0; j < 3; j++) w[yy][j] = __ldg(p + j);
+        }
+#pragma unroll
+        for (int32_t yy = 0; yy < 4; yy++) {
+            float lum[4], blue[4], green[4];
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                float ch[3];
+#pragma unroll
+                for (int c = 0; c < 3; c++) ch[c] = (float)((w[yy][(3 * p + c) >> 2] >> (8 * ((3 * p + c) & 3))) & 255u);
+                lum[p] = eye_lum(__fadd_rn(__fadd_rn(ch[0], ch[1]), ch[2]));
+                blue[p] = chrom ? eye_channel(ch[2]) : 0.0f;
+                green[p] = chrom ? eye_channel(ch[1]) : 0.0f;
             }
-            float r = 0.0f, rb = 0.0f, rg = 0.0f;
-            auto add = [&](int p) {
-                r = __fadd_rn(r, t_lum[ch[3 * p] + ch[3 * p + 1] + ch[3 * p + 2]]);
-                if (chrom) {
-                    rb = __fadd_rn(rb, t_ch[ch[3 * p + 2]]);
-                    rg = __fadd_rn(rg, t_ch[ch[3 * p + 1]]);
-                }
+            // a row of fewer than eight values is summed in order; the mirrored frame's pixel xx is this
+            // segment's 3 - xx
+            auto row = [&](const float (&v)[4]) {
+                const float r0 = fl ? v[3] : v[0], r1 = fl ? v[2] : v[1], r2 = fl ? v[1] : v[2], r3 = fl ? v[0] : v[3];
+                return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(0.0f, r0), r1), r2), r3);
             };
-            if (fl) {                           // the mirrored frame's pixel xx is this segment's 3 - xx
-#pragma unroll
-                for (int xx = 0; xx < 4; xx++) add(3 - xx);
-            } else {
-#pragma unroll
-                for (int xx = 0; xx < 4; xx++) add(xx);
+            s = __fadd_rn(s, row(lum));
+            if (chrom) {
+                sb = __fadd_rn(sb, row(blue));
+                sg = __fadd_rn(sg, row(green));
             }
-            s = __fadd_rn(s, r);
-            sb = __fadd_rn(sb, rb);
-            sg = __fadd_rn(sg, rg);
         }
     } else {
         auto px = [&](int32_t yy, int32_t xx) {
@@ -285,127 +286,246 @@ __device__ __forceinline__ void cell_sums(const EyeArgs& a, const uint8_t* fr, b
         for (int32_t yy = 0; yy < a.cell; yy++) {
             s = __fadd_rn(s, np_row_sum(a.cell, [&](int32_t xx) {
                               const uint8_t* v = px(yy, xx);
-                              return t_lum[v[0] + v[1] + v[2]];
+                              return eye_lum((float)(v[0] + v[1] + v[2]));
                           }));
             if (chrom) {
-                sb = __fadd_rn(sb, np_row_sum(a.cell, [&](int32_t xx) { return t_ch[px(yy, xx)[2]]; }));
-                sg = __fadd_rn(sg, np_row_sum(a.cell, [&](int32_t xx) { return t_ch[px(yy, xx)[1]]; }));
+                sb = __fadd_rn(sb, np_row_sum(a.cell, [&](int32_t xx) { return eye_channel((float)px(yy, xx)[2]); }));
+                sg = __fadd_rn(sg, np_row_sum(a.cell, [&](int32_t xx) { return eye_channel((float)px(yy, xx)[1]); }));
             }
         }
     }
 }
 
+// One thread per (instance, grid cell): luminance, colour grids, high-pass signal (`sig`, the ON half of
+// the state: hp itself; ON is max(hp, 0), OFF max(-hp, 0)) and the delay arms: this frame's into the
+// scratch halves (ON: sig's OFF half; OFF: the integral image's place) and the next frame's into dly.
+// Bound by instruction issue: twenty instructions a pixel.
 template <bool VEC4>
-__global__ void __launch_bounds__(1024) k_eye_fused(const EyeArgs a, const EyeSmem L)
+__global__ void __launch_bounds__(256) k_eye_grid(const EyeArgs a)
 {
-    extern __shared__ __align__(16) unsigned char eye_smem[];
-    const int32_t b = blockIdx.x, cells = L.cells, W1 = a.gw + 1;
-    double* s_con = reinterpret_cast<double*>(eye_smem);
-    float* s_lum = reinterpret_cast<float*>(eye_smem + (size_t)cells * 8 * L.sust);
-    float* s_sig = s_lum + cells;                 // ON, OFF
-    float* s_dly = s_sig + 2 * cells;             // ON, OFF
-    float* s_col = s_dly + 2 * cells;             // blue, green (chromatic only)
-    float* s_ii = s_col + 2 * cells * L.chrom;    // (gh + 1) x (gw + 1) (sustained only)
-    float* t_lum = s_ii + L.ii * L.sust;          // 766 + 256 quotient tables
-    float* t_ch = t_lum + 766;
-    for (int32_t i = threadIdx.x; i < EyeSmem::TAB; i += blockDim.x) {
-        if (i < 766) t_lum[i] = __fdiv_rn(__fdiv_rn((float)i, 3.0f), 255.0f);
-        else t_ch[i - 766] = __fdiv_rn((float)(i - 766), 255.0f);
-    }
-    __syncthreads();
+    const int64_t cells = (int64_t)a.gh * a.gw;
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= (int64_t)a.B * cells) return;
+    const int32_t b = (int32_t)(p / cells), q = (int32_t)(p - (int64_t)b * cells);
+    const int32_t y = q / a.gw, x = q - y * a.gw;
     const bool restart = a.restart[b] != 0, fl = a.flip && a.flip[b];
-    const uint8_t* fr = a.frames + (int64_t)b * a.H * a.W * 3;
+    float* dly = a.dly + (int64_t)b * 2 * cells + q;
+    float lp = a.lp[p], d_on = dly[0], d_off = dly[cells];          // (in flight beside the pixels)
+    float s, sb, sg;
+    cell_sums<VEC4>(a, a.frames + (int64_t)b * a.H * a.W * 3, fl, y, x, a.chromatic != 0, s, sb, sg);
     const float area = (float)(a.cell * a.cell);
-    float* lp_g = a.lp + (int64_t)b * cells;
-    float* dly_g = a.dly + (int64_t)b * 2 * cells;
-    for (int32_t q = threadIdx.x; q < cells; q += blockDim.x) {
-        const int32_t y = q / a.gw, x = q - y * a.gw;
-        float s, sb, sg;
-        cell_sums<VEC4>(a, fr, fl, y, x, t_lum, t_ch, L.chrom != 0, s, sb, sg);
-        const float lum = __fdiv_rn(s, area);
-        s_lum[q] = lum;
-        if (L.chrom) {
-            s_col[q] = __fdiv_rn(sb, area);
-            s_col[cells + q] = __fdiv_rn(sg, area);
-        }
-        float lp = restart ? lum : lp_g[q];
-        lp = __fadd_rn(lp, __fmul_rn(a.a_hp, __fsub_rn(lum, lp)));
-        lp_g[q] = lp;
-        const float hp = __fsub_rn(lum, lp);
-        s_sig[q] = fmaxf(hp, 0.0f);
-        s_sig[cells + q] = fmaxf(-hp, 0.0f);
-        s_dly[q] = restart ? 0.0f : dly_g[q];
-        s_dly[cells + q] = restart ? 0.0f : dly_g[cells + q];
+    const float lum = __fdiv_rn(s, area);
+    a.lum[p] = lum;
+    if (a.chromatic) {
+        a.col[(int64_t)b * 2 * cells + q] = __fdiv_rn(sb, area);
+        a.col[((int64_t)b * 2 + 1) * cells + q] = __fdiv_rn(sg, area);
     }
-    __syncthreads();
-    if (L.sust) {
-        const int32_t t = threadIdx.x;
-        if (t <= a.gw) {                          // padded column t, down the rows
-            float c = 0.0f;
-            s_ii[t] = 0.0f;
-            for (int32_t i = 1; i <= a.gh; i++) {
-                c = __fadd_rn(c, t == 0 ? 0.0f : s_lum[(i - 1) * a.gw + t - 1]);
-                s_ii[i * W1 + t] = c;
+    if (restart) {
+        lp = lum;
+        d_on = d_off = 0.0f;
+    }
+    lp = __fadd_rn(lp, __fmul_rn(a.a_hp, __fsub_rn(lum, lp)));
+    a.lp[p] = lp;
+    const float hp = __fsub_rn(lum, lp);
+    a.sig[(int64_t)b * 2 * cells + q] = hp;
+    a.sig[((int64_t)b * 2 + 1) * cells + q] = d_on;
+    a.ii[(int64_t)b * (a.gh + 1) * (a.gw + 1) + q] = d_off;
+    dly[0] = __fadd_rn(d_on, __fmul_rn(a.a_d, __fsub_rn(fmaxf(hp, 0.0f), d_on)));
+    dly[cells] = __fadd_rn(d_off, __fmul_rn(a.a_d, __fsub_rn(fmaxf(-hp, 0.0f), d_off)));
+}
+
+// The neurons [blockIdx.x * run, ...) of instance blockIdx.y. The block keeps the instance's grids in shared
+// memory (a neuron gathers up to four cells of them), forms the integral image there (every block of an
+// instance for itself: sharing it would cost a launch), and takes the neurons in chunks sorted by the
+// kind of their channel, so that a warp works on one kind; their rates go out in neuron order through
+// shared memory. Gathered from L1 and unsorted, 64 x 12,246 neurons took 25.7 us, now 16.5; what bounds it is
+// instruction issue (~200 a neuron, 60 of them the sort).
+constexpr int EYE_THREADS = 1024, EYE_UNROLL = 4, EYE_CHUNK = EYE_THREADS * EYE_UNROLL;
+
+struct EyeSmem {                                                   // offsets in floats
+    int32_t hp, on, off, lum, ii, col, rate, order, total;
+    EyeSmem() = default;
+    EyeSmem(int32_t cells, int32_t ii_cells, bool sust, bool chrom)
+    {
+        hp = 0;
+        on = hp + cells;
+        off = on + cells;
+        lum = off + cells;
+        ii = lum + (sust ? cells : 0);
+        col = ii + (sust ? ii_cells : 0);
+        rate = col + (chrom ? 2 * cells : 0);
+        order = rate + EYE_CHUNK;
+        total = order + EYE_CHUNK;
+    }
+};
+
+// running sums of n values `stride` apart, eight loaded at a time
+__device__ __forceinline__ void running_sum(float* v, int32_t n, int32_t stride)
+{
+    float c = 0.0f;
+    int32_t i = 0;
+    for (; i + 8 <= n; i += 8) {
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = v[(i + u) * stride];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[(i + u) * stride] = c = __fadd_rn(c, x[u]);
+    }
+    for (; i < n; i++) v[i * stride] = c = __fadd_rn(c, v[i * stride]);
+}
+
+__global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, const EyeSmem S, int32_t run)
+{
+    extern __shared__ float sm[];
+    __shared__ int32_t s_kind[4];                                  // neurons of each kind in the chunk
+    const int32_t b = blockIdx.y, W1 = a.gw + 1, tid = threadIdx.x, lane = tid & 31;
+    const int32_t cells = a.gh * a.gw;
+    float *s_hp = sm + S.hp, *s_on = sm + S.on, *s_off = sm + S.off, *s_lum = sm + S.lum, *s_ii = sm + S.ii;
+    float *s_col = sm + S.col, *s_rate = sm + S.rate;
+    uint32_t* s_order = reinterpret_cast<uint32_t*>(sm + S.order); // per sorted place: entry | channel << 12 | visible << 16
+    const bool sust = a.sustained != 0.0;
+    const int32_t k1 = min(a.n_cells, (int32_t)(blockIdx.x + 1) * run);
+    // a chunk's neurons, loaded ahead (the first one's beside the grids): cell (-1: out of range, or no neuron),
+    // channel and visibility, ext slot
+    int32_t cell[EYE_UNROLL], chan[EYE_UNROLL], slot[EYE_UNROLL];
+    auto fetch = [&](int32_t first) {
+#pragma unroll
+        for (int u = 0; u < EYE_UNROLL; u++) {
+            const int32_t k = first + tid + u * EYE_THREADS;
+            cell[u] = -1;
+            chan[u] = slot[u] = 0;
+            if (k >= k1) continue;
+            const int32_t x = __ldg(a.gx + k), y = __ldg(a.gy + k), c = __ldg(a.chan + k);
+            slot[u] = __ldg(a.slot + k);
+            chan[u] = c | ((int32_t)(__ldg(a.visible + k) != 0) << 4);
+            if (x >= 0 && x < a.gw && y >= 0 && y < a.gh && c < EYE_CHANNELS && slot[u] >= 0 && slot[u] < a.n_ext) cell[u] = y * a.gw + x;
+        }
+    };
+    fetch(blockIdx.x * run);
+    {
+        const float* hp = a.sig + (int64_t)b * 2 * cells;
+        const float* off = a.ii + (int64_t)b * (a.gh + 1) * W1;
+        const float* lum = a.lum + (int64_t)b * cells;
+        const float* col = a.col + (int64_t)b * 2 * cells;
+        for (int32_t q = tid; q < cells; q += EYE_THREADS) {
+            s_hp[q] = hp[q];
+            s_on[q] = hp[cells + q];
+            s_off[q] = off[q];
+            if (sust) {
+                const float l = lum[q];
+                const int32_t y = q / a.gw, x = q - y * a.gw;
+                s_lum[q] = l;
+                s_ii[(y + 1) * W1 + x + 1] = l;
+            }
+            if (a.chromatic) {
+                s_col[q] = col[q];
+                s_col[cells + q] = col[cells + q];
             }
         }
-        __syncthreads();
-        if (t <= a.gh) {                          // row t, along the columns
-            float* r = s_ii + t * W1;
-            float c = r[0];
-            for (int32_t j = 1; j <= a.gw; j++) {
-                c = __fadd_rn(c, r[j]);
-                r[j] = c;
+        if (sust) {                                                // a border of zeros
+            for (int32_t t = tid; t <= a.gw; t += EYE_THREADS) s_ii[t] = 0.0f;
+            for (int32_t t = tid; t <= a.gh; t += EYE_THREADS) s_ii[t * W1] = 0.0f;
+            __syncthreads();
+            for (int32_t t = tid; t <= a.gw; t += EYE_THREADS) running_sum(s_ii + t, a.gh + 1, W1);      // down the rows,
+            __syncthreads();
+            for (int32_t t = tid; t <= a.gh; t += EYE_THREADS) running_sum(s_ii + t * W1, W1, 1);        // then along them
+        }
+    }
+    for (int32_t first = blockIdx.x * run; first < k1; first += EYE_CHUNK) {
+        if (tid < 4) s_kind[tid] = 0;
+        __syncthreads();                                           // (the grids are in place, the last chunk is out)
+        // the neurons' places, sorted by kind: ballots count a warp's, one atomic per kind and warp reserves theirs
+        int32_t kind[EYE_UNROLL], at[EYE_UNROLL], mine = 0;
+#pragma unroll
+        for (int u = 0; u < EYE_UNROLL; u++) {
+            const int32_t c = chan[u] & 15;
+            kind[u] = cell[u] < 0 ? -1 : c < EYE_ON_TRANSIENT ? 0 : c <= EYE_OFF_TRANSIENT ? 1 : c <= EYE_OFF_SUSTAINED ? 2 : 3;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            int32_t n = 0;
+#pragma unroll
+            for (int u = 0; u < EYE_UNROLL; u++) {
+                const uint32_t m = __ballot_sync(0xffffffffu, kind[u] == i);
+                if (kind[u] == i) at[u] = n + __popc(m & ((1u << lane) - 1u));
+                n += __popc(m);
             }
+            if (lane == i) mine = n;
+        }
+        int32_t base = 0;
+        if (lane < 4 && mine) base = atomicAdd(&s_kind[lane], mine);
+#pragma unroll
+        for (int u = 0; u < EYE_UNROLL; u++) {
+            const int32_t from = __shfl_sync(0xffffffffu, base, kind[u] & 3);
+            if (kind[u] >= 0) at[u] += from;
         }
         __syncthreads();
-        const int32_t rr = a.surround;
-        for (int32_t q = threadIdx.x; q < cells; q += blockDim.x) {
+        int32_t count = 0, before[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            before[i] = count;
+            count += s_kind[i];
+        }
+#pragma unroll
+        for (int u = 0; u < EYE_UNROLL; u++)
+            if (kind[u] >= 0) {
+                const int32_t e = tid + u * EYE_THREADS;
+                const int32_t bf = kind[u] == 0 ? before[0] : kind[u] == 1 ? before[1] : kind[u] == 2 ? before[2] : before[3];
+                s_order[bf + at[u]] = (uint32_t)e | ((uint32_t)chan[u] << 12);
+                s_rate[e] = __int_as_float(cell[u]);               // its cell, until its rate takes the place
+            }
+        __syncthreads();
+        // (in turn, so that the code of one neuron is not unrolled four times)
+#pragma unroll 1
+        for (int32_t at_e = tid; at_e < count; at_e += EYE_THREADS) {
+            const uint32_t o = s_order[at_e];
+            const int32_t e = (int32_t)(o & (EYE_CHUNK - 1)), c = (int32_t)((o >> 12) & 15u), q = __float_as_int(s_rate[e]);
             const int32_t y = q / a.gw, x = q - y * a.gw;
-            const int32_t y0 = min(max(y - rr, 0), a.gh), y1 = min(max(y + rr + 1, 0), a.gh);
-            const int32_t x0 = min(max(x - rr, 0), a.gw), x1 = min(max(x + rr + 1, 0), a.gw);
-            const float num = __fadd_rn(__fsub_rn(__fsub_rn(s_ii[y1 * W1 + x1], s_ii[y0 * W1 + x1]), s_ii[y1 * W1 + x0]),
-                                        s_ii[y0 * W1 + x0]);
-            const double sur = __ddiv_rn((double)num, (double)((int64_t)(y1 - y0) * (x1 - x0)));
-            s_con[q] = __dsub_rn((double)s_lum[q], sur);
+            float r = 0.0f;
+            if (c < EYE_ON_TRANSIENT) {
+                const int32_t dir = c & 3, sh = a.shift;
+                const float sgn = (c >> 2) ? -1.0f : 1.0f;         // (a sign change is exact)
+                const float* dl = (c >> 2) ? s_off : s_on;
+                float corr = 0.0f;
+                if (dir < 2 ? x < a.gw - sh : y < a.gh - sh) {
+                    const int32_t q1 = dir < 2 ? q + sh : q + sh * a.gw;
+                    const float s0 = fmaxf(sgn * s_hp[q], 0.0f), s1 = fmaxf(sgn * s_hp[q1], 0.0f);
+                    corr = __fsub_rn(__fmul_rn(dl[q], s1), __fmul_rn(s0, dl[q1]));
+                }
+                r = (dir & 1) ? fmaxf(-corr, 0.0f) : fmaxf(corr, 0.0f);
+            } else if (c <= EYE_OFF_TRANSIENT) {
+                const float h = s_hp[q];
+                r = __fdiv_rn(__fmul_rn(a.transient_f, fmaxf(c == EYE_ON_TRANSIENT ? h : -h, 0.0f)), a.gain_f);
+            } else if (c <= EYE_OFF_SUSTAINED) {
+                if (sust) {
+                    const int32_t rr = a.surround;
+                    const int32_t y0 = min(max(y - rr, 0), a.gh), y1 = min(max(y + rr + 1, 0), a.gh);
+                    const int32_t x0 = min(max(x - rr, 0), a.gw), x1 = min(max(x + rr + 1, 0), a.gw);
+                    const float num = __fadd_rn(__fsub_rn(__fsub_rn(s_ii[y1 * W1 + x1], s_ii[y0 * W1 + x1]), s_ii[y1 * W1 + x0]),
+                                                s_ii[y0 * W1 + x0]);
+                    const double sur = __ddiv_rn((double)num, (double)((int64_t)(y1 - y0) * (x1 - x0)));
+                    const double con = __dsub_rn((double)s_lum[q], sur);
+                    const double m = c == EYE_ON_SUSTAINED ? fmax(con, 0.0) : fmax(-con, 0.0);
+                    r = __double2float_rn(__ddiv_rn(__dmul_rn(a.sustained, m), a.gain));
+                }
+            } else if (a.chromatic) {
+                r = __fdiv_rn(__fmul_rn(a.chromatic_f, s_col[(c - EYE_BLUE) * cells + q]), a.gain_f);
+            }
+            if (!((o >> 16) & 1u)) r = 0.0f;
+            s_rate[e] = __fmul_rn(a.max_rate, fminf(fmaxf(__fmul_rn(a.gain_f, r), 0.0f), 1.0f));
         }
         __syncthreads();
-    }
-    for (int32_t k = threadIdx.x; k < a.n_cells; k += blockDim.x) {
-        const int32_t c = __ldg(a.chan + k), x = __ldg(a.gx + k), y = __ldg(a.gy + k), s = __ldg(a.slot + k);
-        if (x < 0 || x >= a.gw || y < 0 || y >= a.gh || c >= EYE_CHANNELS || s < 0 || s >= a.n_ext) continue;
-        const int32_t q = y * a.gw + x;
-        float r = 0.0f;
-        if (c < EYE_ON_TRANSIENT) {
-            const int32_t pol = c >> 2, dir = c & 3, sh = a.shift;
-            const float* sg = s_sig + pol * cells;
-            const float* dl = s_dly + pol * cells;
-            float corr = 0.0f;
-            if (dir < 2) {
-                if (x < a.gw - sh) corr = __fsub_rn(__fmul_rn(dl[q], sg[q + sh]), __fmul_rn(sg[q], dl[q + sh]));
-            } else if (y < a.gh - sh) {
-                const int32_t q1 = q + sh * a.gw;
-                corr = __fsub_rn(__fmul_rn(dl[q], sg[q1]), __fmul_rn(sg[q], dl[q1]));
-            }
-            r = (dir & 1) ? fmaxf(-corr, 0.0f) : fmaxf(corr, 0.0f);
-        } else if (c <= EYE_OFF_TRANSIENT) {
-            r = __fdiv_rn(__fmul_rn(a.transient_f, s_sig[(c - EYE_ON_TRANSIENT) * cells + q]), a.gain_f);
-        } else if (c <= EYE_OFF_SUSTAINED) {
-            if (L.sust) {
-                const double con = s_con[q];
-                const double m = c == EYE_ON_SUSTAINED ? fmax(con, 0.0) : fmax(-con, 0.0);
-                r = __double2float_rn(__ddiv_rn(__dmul_rn(a.sustained, m), a.gain));
-            }
-        } else if (L.chrom) {
-            r = __fdiv_rn(__fmul_rn(a.chromatic_f, s_col[(c - EYE_BLUE) * cells + q]), a.gain_f);
+#pragma unroll
+        for (int u = 0; u < EYE_UNROLL; u++) {
+            if (kind[u] < 0) continue;
+            const int32_t e = tid + u * EYE_THREADS;
+            const float rate = s_rate[e];
+            if (a.rates) a.rates[(int64_t)b * a.n_cells + first + e] = rate;
+            a.p_ext[(int64_t)b * a.n_ext + slot[u]] = __fmul_rn(rate, a.p_scale);
         }
-        if (!__ldg(a.visible + k)) r = 0.0f;
-        const float rate = __fmul_rn(a.max_rate, fminf(fmaxf(__fmul_rn(a.gain_f, r), 0.0f), 1.0f));
-        if (a.rates) a.rates[(int64_t)b * a.n_cells + k] = rate;
-        a.p_ext[(int64_t)b * a.n_ext + s] = __fmul_rn(rate, a.p_scale);
+        if (first + EYE_CHUNK < k1) fetch(first + EYE_CHUNK);
     }
-    for (int32_t q = threadIdx.x; q < 2 * cells; q += blockDim.x)
-        dly_g[q] = __fadd_rn(s_dly[q], __fmul_rn(a.a_d, __fsub_rn(s_sig[q], s_dly[q])));
-    if (threadIdx.x == 0) a.restart[b] = 0;
+    if (blockIdx.x == 0 && tid == 0) a.restart[b] = 0;
 }
 
 }  // namespace fb

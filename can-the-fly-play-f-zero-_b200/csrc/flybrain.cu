@@ -747,20 +747,27 @@ extern "C" int fb_motion_eye(fb_brain* h, const uint8_t* frames, int32_t H, int3
     a.n_cells = n_cells; a.gx = gx; a.gy = gy; a.chan = chan; a.visible = visible; a.slot = slot;
     a.p_ext = h->p_ext; a.n_ext = (int32_t)h->n_ext; a.rates = rates;
     cudaStream_t st = (cudaStream_t)stream;
-    const EyeSmem L{gh * gw, (gh + 1) * (gw + 1), a.chromatic ? 1 : 0, ep->sustained_gain != 0.0 ? 1 : 0};
-    const size_t smem = L.bytes();
-    const bool fits = smem <= 227 * 1024;
-    if (ep->kernels == 1 && !fits) return fail(FB_ERR_ARG, "eye grid too large for the one-block-per-instance kernel");
-    if (ep->kernels != 2 && fits) {
-        const bool vec4 = ep->cell == 4 && W % 4 == 0 && ((uintptr_t)frames & 3) == 0;
-        const void* fn = vec4 ? (const void*)k_eye_fused<true> : (const void*)k_eye_fused<false>;
-        CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (vec4)
-            k_eye_fused<true><<<h->B, 1024, smem, st>>>(a, L);
-        else
-            k_eye_fused<false><<<h->B, 1024, smem, st>>>(a, L);
+    // kernels 1 promises a grid that one block could hold in shared memory (luminance, signals, delay arms,
+    // colours, integral image, contrast); the two-launch form needs the integral image there
+    const int64_t grid = (int64_t)gh * gw, ii = (int64_t)(gh + 1) * (gw + 1);
+    const bool sust = ep->sustained_gain != 0.0;
+    const int64_t block = grid * (8 * sust + 4 * (5 + 2 * a.chromatic)) + ii * 4 * sust + (766 + 256) * 4;
+    if (ep->kernels == 1 && block > 227 * 1024)
+        return fail(FB_ERR_ARG, "eye grid too large for the one-block-per-instance kernel");
+    const int64_t floats = grid * (3 + sust + 2 * a.chromatic) + ii * sust + 2 * EYE_CHUNK;
+    if (ep->kernels != 2 && floats * 4 <= 227 * 1024 && h->B <= 65535) {
+        const unsigned blocks = (unsigned)((cells + 255) / 256);
+        if (ep->cell == 4 && W % 4 == 0 && ((uintptr_t)frames & 3) == 0) k_eye_grid<true><<<blocks, 256, 0, st>>>(a);
+        else k_eye_grid<false><<<blocks, 256, 0, st>>>(a);
         CU(cudaGetLastError());
-        h->launches += 1;
+        // blocks per instance: enough to fill the SMs once, at least EYE_THREADS neurons each
+        const EyeSmem S((int32_t)grid, (int32_t)ii, sust, a.chromatic != 0);
+        const int32_t per = std::max(1, std::min(h->sm_count / h->B, (n_cells + EYE_THREADS - 1) / EYE_THREADS));
+        const int32_t run = std::max(1, (n_cells + per - 1) / per);
+        CU(cudaFuncSetAttribute(k_eye_neurons, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total * 4));
+        k_eye_neurons<<<dim3((unsigned)per, (unsigned)h->B), EYE_THREADS, (size_t)S.total * 4, st>>>(a, S, run);
+        CU(cudaGetLastError());
+        h->launches += 2;
         return FB_OK;
     }
     int launches = 2;

@@ -3,7 +3,7 @@
 ``BatchMotionEye`` is the batched drop-in for ``flyzero.vision.MotionEye`` (flyzero/vision.py:
 64-191): one eye per instance, the same neurons in the same order (``idx``, ``px``, ``py``,
 ``side``), the same float32 filter state per instance, and ``see`` computes every instance's rates
-from a device batch of frames in one kernel launch (fb_motion_eye), writing them straight into
+from a device batch of frames in one call (fb_motion_eye), writing them straight into
 the brain's Poisson probabilities (``p_ext``) — the reference computes one eye per fly on the host
 and hands the rates to ``set_input``.
 
@@ -162,8 +162,8 @@ def _p(t):
 
 class BatchMotionEye:
     """One ``MotionEye`` per instance of ``brain``; ``see`` drives the eye neurons' Poisson input.
-    ``kernels``: "fused" runs each instance's eye in one thread block with its grid in shared
-    memory (one launch), "split" runs four grid-wide kernels, "auto" the first when it fits."""
+    ``kernels``: "fused" runs a grid kernel and a neuron kernel that keeps the instance's grids in
+    shared memory, "split" runs four grid-wide kernels, "auto" the first when it fits."""
 
     def __init__(self, brain, conn, frame_shape, params: MotionParams | None = None, eye_layout: EyeLayout | None = None,
                  kernels: str = "auto"):
