@@ -90,8 +90,9 @@ __global__ void k_reset(Real* v, Real* g, int8_t* ref, void* acc, int32_t n_slot
         const int64_t a = (int64_t)b * n_pad + (p - (int64_t)b * n);
         for (int32_t k = 0; k < n_slots; k++) {
             const int64_t o = (int64_t)k * B * n_pad + a;
-            if (acc_bytes == 4) ((int32_t*)acc)[o] = 0;
-            else ((int64_t*)acc)[o] = 0;
+            if (acc_bytes == 8) ((int64_t*)acc)[o] = 0;
+            else if (acc_bytes == 4) ((int32_t*)acc)[o] = 0;
+            else if (!(o & 1)) ((int32_t*)acc)[o >> 1] = 0;      // the word of this pair and the next (rows are even)
         }
     }
     const int64_t ptotal = (int64_t)R * B * n_ppost;
@@ -99,6 +100,36 @@ __global__ void k_reset(Real* v, Real* g, int8_t* ref, void* acc, int32_t n_slot
         const int32_t b = (int32_t)((p / n_ppost) % B);
         if (fly_mask && !fly_mask[b]) continue;
         pring[p] = 0;
+    }
+}
+
+// Every neuron's sum of |count| over its incoming entries, then the largest of them into sums[n]
+__global__ void k_input_sums(const int32_t* col, const int16_t* cnt, int64_t entries, unsigned long long* sums)
+{
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < entries; k += (int64_t)gridDim.x * blockDim.x)
+        if (cnt[k] != 0) atomicAdd(sums + col[k], (unsigned long long)abs((int)cnt[k]));
+}
+__global__ void k_largest(unsigned long long* sums, int64_t n)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        atomicMax(sums + n, sums[i]);
+}
+
+// The accumulators from 32 to 16 bits (two pairs to a word) or back, when a run starts on the other engine;
+// those left behind are zero
+__global__ void k_repack(int32_t* wide, int32_t* narrow, int64_t words, bool to_narrow)
+{
+    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (int64_t)gridDim.x * blockDim.x) {
+        int2* p = reinterpret_cast<int2*>(wide) + w;
+        if (to_narrow) {
+            const int2 x = *p;
+            narrow[w] = (int32_t)(((uint32_t)x.y << 16) + (uint32_t)x.x);
+            if (x.x | x.y) *p = make_int2(0, 0);
+        } else {
+            const int32_t x = narrow[w];
+            *p = make_int2(lo16(x), hi16(x));
+            if (x) narrow[w] = 0;
+        }
     }
 }
 
@@ -162,7 +193,9 @@ struct fb_brain {
     HostCsr hc;                       // host copy of the CSR for re-planning the plastic entries
     PlasticPlan plastic;              // current plastic plan
     // delay line
-    void* acc = nullptr;          // [n_slots][B][n_pad]
+    void* acc = nullptr;          // [n_slots][B][n_pad] int32 or int64
+    void* acc16 = nullptr;        // the same in 16 bits for the persistent engine, where every input sum fits
+    bool live16 = false;          // the input in flight is in acc16 (acc is zero), else in acc (acc16 is zero)
     int32_t n_slots = 2;
     int32_t epoch = 1;            // persistent engine: steps per grid barrier
     int64_t pushed_until = 1;     // the arrivals of every tick < pushed_until are in acc
@@ -219,7 +252,7 @@ struct fb_brain {
     {
         DevState S{};
         S.v = v; S.g = g; S.ref = ref; S.pw = pw; S.ext_idx = ext_idx; S.n_ext = (int32_t)n_ext;
-        S.p_ext = p_ext; S.bias_ext = bias_ext; S.acc = acc; S.n_slots = n_slots; S.pring = pring;
+        S.p_ext = p_ext; S.bias_ext = bias_ext; S.acc = live16 ? acc16 : acc; S.n_slots = n_slots; S.pring = pring;
         S.items = items; S.item_count = item_count; S.cap_c = cap_c; S.group = list_group;
         S.n_groups = n_groups; S.reset_tick = reset_tick;
         S.stop_tick = stop_tick; S.err = err_d; S.seed = seed;
@@ -234,7 +267,7 @@ int free_all(fb_brain* h)
 {
     void* ptrs[] = {h->rowptr, h->col, h->cnt, h->wfx, h->pl_rowptr, h->pl_pidx, h->pl_q0, h->ppost_of, h->pw, h->w0,
                     h->pl_pre, h->pl_post, h->ppost_neuron,
-                    h->v, h->g, h->ref, h->ext_idx, h->p_ext, h->bias_ext, h->acc, h->pring,
+                    h->v, h->g, h->ref, h->ext_idx, h->p_ext, h->bias_ext, h->acc, h->acc16, h->pring,
                     h->items, h->item_count, h->reset_tick, h->stop_tick, h->fly_mask, h->bar, h->abort_flag,
                     h->ext_tab, h->ext_off, h->colptr, h->cpre, h->ccnt, h->cwfx, h->masks};
     for (void* p : ptrs)
@@ -320,6 +353,25 @@ int build_ext_table(fb_brain* h)
     int rc = upload(&h->ext_tab, tab, &h->bytes);
     if (rc) return rc;
     return upload(&h->ext_off, off, &h->bytes);
+}
+
+// No step's input of any neuron can exceed `out` in size: the connectome's largest input sum (counts only)
+int largest_input(fb_brain* h, int64_t* out)
+{
+    unsigned long long* sums = nullptr;
+    unsigned long long top = 0;
+    CU(cudaMalloc(&sums, (size_t)(h->n + 1) * sizeof(*sums)));
+    cudaError_t e = cudaMemset(sums, 0, (size_t)(h->n + 1) * sizeof(*sums));
+    if (e == cudaSuccess) {
+        k_input_sums<<<h->sm_count * 8, 256>>>(h->col, h->cnt, h->nnz_pad, sums);
+        k_largest<<<(unsigned)std::min<int64_t>((h->n + 255) / 256, h->sm_count), 256>>>(sums, h->n);
+        h->launches += 2;
+        e = cudaMemcpy(&top, sums + h->n, sizeof(top), cudaMemcpyDeviceToHost);
+    }
+    cudaFree(sums);
+    CU(e);
+    *out = (int64_t)top;
+    return FB_OK;
 }
 
 int dispatch_step(fb_brain* h, const StepArgs& A, bool raster, bool record, cudaStream_t st);
@@ -421,11 +473,21 @@ extern "C" int fb_create(const fb_params* P, const int64_t* indptr, const int32_
     h->plan = plan_persistent(h->n, h->n_pad, h->B, h->f64 != 0, h->n_ref, h->n_delay, dev_sms2, h->device);
     // the persistent engine runs epochs of K steps between grid barriers: the spikes of an epoch, listed
     // in the next one, arrive three epochs later at the earliest when 3K <= n_delay; 2K accumulator slots
-    h->epoch = h->plan.group > 0 ? persistent_epoch(h->plan, h->n_pad, h->n_delay, (int)ab) : 1;
+    // its accumulators are 16 bits wide if no neuron's input can leave them in any step (all its presynaptic
+    // neurons firing at once): half the bytes to read, clear and keep in L2
+    int64_t largest = 0;
+    if (h->plan.group > 0 && h->acc_mode == 0) TRY(largest_input(h, &largest));
+    const bool narrow = h->plan.group > 0 && h->acc_mode == 0 && largest <= INT16_MAX;
+    h->epoch = h->plan.group > 0 ? persistent_epoch(h->plan, h->n_pad, h->n_delay, narrow ? 2 : (int)ab) : 1;
     h->n_slots = 2 * h->epoch;
     h->R_pl = h->R = h->n_delay + h->epoch;
     TRY(dalloc((char**)&h->acc, nbp * ab * h->n_slots, tb));
     CU(cudaMemset(h->acc, 0, nbp * ab * h->n_slots));
+    if (narrow) {
+        TRY(dalloc((char**)&h->acc16, nbp * 2 * h->n_slots, tb));
+        CU(cudaMemset(h->acc16, 0, nbp * 2 * h->n_slots));
+        h->live16 = true;             // (all zero: nothing to carry over)
+    }
     h->list_group = h->plan.group > 0 ? h->plan.group : h->B;
     h->n_groups = (h->B + h->list_group - 1) / h->list_group;
     TRY(install_plastic(h, pos));
@@ -563,12 +625,12 @@ extern "C" int fb_reset(fb_brain* h, const int32_t* flies, int32_t n_flies, void
     }
     const int64_t total = (int64_t)h->B * h->n;
     const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)h->sm_count * 16);
-    const int ab = h->acc_mode == 0 ? 4 : 8;
+    const int ab = h->live16 ? 2 : h->acc_mode == 0 ? 4 : 8;
     if (h->f64)
         k_reset<double><<<blocks, 256, 0, st>>>((double*)h->v, (double*)h->g, h->ref, h->acc, h->n_slots, ab, h->pring,
                                                 h->R_pl, h->B, h->n, h->n_pad, h->n_ppost, mask, h->params.v_rest);
     else
-        k_reset<float><<<blocks, 256, 0, st>>>((float*)h->v, (float*)h->g, h->ref, h->acc, h->n_slots, ab, h->pring,
+        k_reset<float><<<blocks, 256, 0, st>>>((float*)h->v, (float*)h->g, h->ref, h->live16 ? h->acc16 : h->acc, h->n_slots, ab, h->pring,
                                                h->R_pl, h->B, h->n, h->n_pad, h->n_ppost, mask, (float)h->params.v_rest);
     CU(cudaGetLastError());
     h->launches += 1;
@@ -932,7 +994,16 @@ extern "C" int fb_run(fb_brain* h, int32_t steps, int32_t* counts_out, const uin
     int engine = h->engine;
     if (engine == FB_ENGINE_AUTO)
         engine = (h->plan.group > 0 && !h->f64 && h->prop == FB_PROP_PUSH) ? FB_ENGINE_PERSISTENT : FB_ENGINE_STEP;
-    if (engine == FB_ENGINE_PERSISTENT && h->plan.group > 0 && !h->f64) {
+    const bool persistent = engine == FB_ENGINE_PERSISTENT && h->plan.group > 0 && !h->f64;
+    if (h->acc16 && h->live16 != persistent) {                // the input in flight follows the engine
+        const int64_t accs = (int64_t)h->n_slots * h->B * h->n_pad / 2;
+        k_repack<<<(unsigned)std::min<int64_t>((accs + 255) / 256, (int64_t)h->sm_count * 16), 256, 0, st>>>(
+            (int32_t*)h->acc, (int32_t*)h->acc16, accs, persistent);
+        CU(cudaGetLastError());
+        h->launches += 1;
+        h->live16 = persistent;
+    }
+    if (persistent) {
         h->masks_dirty = h->masks != nullptr;     // no spike masks recorded for these steps
         PersistArgs P{};
         P.t0 = h->t; P.step0 = h->step_no; P.steps = steps; P.kicks = kicks; P.words = words;
@@ -943,7 +1014,7 @@ extern "C" int fb_run(fb_brain* h, int32_t steps, int32_t* counts_out, const uin
         P.epoch = h->epoch;
         P.barrier_cycles = h->barrier_cycles;
         CU(cudaMemsetAsync(h->abort_flag, 0, sizeof(int32_t), st));
-        int rc = launch_persistent(h->plan, h->net(), h->state(), P, h->acc_mode, h->n_pl > 0, kicks != nullptr, record,
+        int rc = launch_persistent(h->plan, h->net(), h->state(), P, h->live16 ? 2 : h->acc_mode == 0 ? 4 : 8, h->n_pl > 0, kicks != nullptr, record,
                                    st);
         if (rc) return fail(FB_ERR_CUDA, "persistent launch: %s", cudaGetErrorString((cudaError_t)rc));
         h->launches += h->plan.launches_per_run;

@@ -19,12 +19,14 @@
 // The listing and pushing warps take tiles too when they are done. One grid barrier ends an epoch;
 // between arriving at it and waiting for it a CTA draws the next epoch's Poisson kicks.
 //
-// What bounds an epoch (16 instances of 138,639 neurons, K = 4: 22 us, against 28 us for a step-by-step
-// kernel with the same epochs): the advance reads 35 MB of accumulators from L2 and the pushes reduce
-// 0.9 M entries into them, each ~10 us alone and 18 us together; the barrier takes 3 us. Advancing an
-// epoch at a time takes the state's shared-memory traffic (22 B per pair and step) and three
-// CTA-level barriers out of every step. 512 threads: with 128 registers each nothing of the advance
-// is spilled; at 1,024 threads its spills, behind the queued reductions, made the epoch 34 us.
+// What bounds an epoch (16 instances of 138,639 neurons, K = 6: 27 us or 4.5 us per step, against 7.0 for
+// a step-by-step kernel): the advance reads 27 MB of accumulators from L2 and the pushes reduce 1.4 M
+// entries into them, each about half of the 22 us they take together; the barrier takes 3-4 us.
+// Advancing an epoch at a time takes the state's shared-memory traffic (22 B per pair and step) and
+// three CTA-level barriers out of every step. 512 threads: with 128 registers each nothing of the
+// advance is spilled; at 1,024 threads its spills, behind the queued reductions, made an epoch of 4
+// steps 34 us instead of 22, and a routine called from the advance that needs more than half of the
+// registers does the same (advance_pairs with two quads per lane group: 40 us per 6 steps).
 //
 // Every wait is bounded: after ~4 s a CTA raises the timeout flag and every CTA returns (the others
 // read the flag in the grid barrier).
@@ -42,7 +44,7 @@ constexpr long long BARRIER_TIMEOUT_CYCLES = 8000000000LL;   // ~4 s at 1.9 GHz
 constexpr int MAX_EPOCH = 6;            // steps per epoch at most
 constexpr int K_BITS = 18;              // bits of a local pair index (per < 2^18)
 
-constexpr int PUSH_WARPS = 4;                              // warps that scatter arriving items ...
+constexpr int PUSH_WARPS = 5;                              // warps that scatter arriving items ...
 constexpr int LIST_WARPS = 2;                              // ... and that list the previous epoch's spikes
 constexpr int PUSH_THREADS = 32 * PUSH_WARPS;
 constexpr int LIST_THREADS = 32 * LIST_WARPS;
@@ -88,8 +90,27 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p)
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ int32_t ld_cg(const int32_t* p) { return __ldcg(p); }
-__device__ __forceinline__ int64_t ld_cg(const int64_t* p) { return __ldcg(reinterpret_cast<const long long*>(p)); }
+// one pair's accumulator: its value, and the word that holds it cleared
+__device__ __forceinline__ int32_t* word_of(int16_t* p) { return reinterpret_cast<int32_t*>((uintptr_t)p & ~(uintptr_t)3); }
+__device__ __forceinline__ int32_t ld_acc(int32_t* p) { return __ldcg(p); }
+__device__ __forceinline__ int64_t ld_acc(int64_t* p) { return __ldcg(reinterpret_cast<const long long*>(p)); }
+__device__ __forceinline__ int32_t ld_acc(int16_t* p)
+{
+    const int32_t w = __ldcg(word_of(p)), lo = (int32_t)(int16_t)w;
+    return ((uintptr_t)p & 2) ? (w - lo) >> 16 : lo;
+}
+template <typename T> __device__ __forceinline__ void clear_acc(T* p) { *p = 0; }
+__device__ __forceinline__ void clear_acc(int16_t* p) { *word_of(p) = 0; }
+// the reduction of one entry into its target's accumulator
+__device__ __forceinline__ void red_acc(int32_t* p, int32_t w) { red_add(p, w); }
+__device__ __forceinline__ void red_acc(int64_t* p, int64_t w) { red_add(p, w); }
+__device__ __forceinline__ void red_acc(int16_t* p, int32_t w)
+{
+    red_add(word_of(p), (int32_t)((uint32_t)w << (8 * ((uint32_t)(uintptr_t)p & 2u))));
+}
+// what a connectome entry adds, and what a pair's accumulator holds
+template <typename AccT> struct SumOf { using T = AccT; };
+template <> struct SumOf<int16_t> { using T = int32_t; };
 __device__ __forceinline__ int ld_volatile_i32(const int32_t* p) { return *reinterpret_cast<const volatile int32_t*>(p); }
 
 __device__ __forceinline__ long long* trace_at(const PersistArgs& A, int32_t s, int slot)
@@ -212,7 +233,21 @@ struct Acc4l {
     }
     __device__ __forceinline__ int64_t at(int j) const { return j == 0 ? a.x : j == 1 ? a.y : j == 2 ? b.x : b.y; }
 };
+// 16-bit accumulators, two pairs to a 32-bit word: a pair's count is added at its half of the word
+// (w << 16 for the odd pair), so the word is S_hi * 2^16 + S_lo mod 2^32, which determines both sums as
+// long as each fits in 16 signed bits (fb_create checks the connectome's largest input sum).
+__device__ __forceinline__ int32_t lo16(int32_t w) { return (int32_t)(int16_t)w; }
+__device__ __forceinline__ int32_t hi16(int32_t w) { return (w - lo16(w)) >> 16; }
+struct Acc4s {
+    int2 a;
+    __device__ __forceinline__ void load(const int16_t* p) { a = __ldcg(reinterpret_cast<const int2*>(p)); }
+    __device__ __forceinline__ void zero() { a = make_int2(0, 0); }
+    __device__ __forceinline__ bool any() const { return (a.x | a.y) != 0; }
+    __device__ __forceinline__ static void clear(int16_t* p) { *reinterpret_cast<int2*>(p) = make_int2(0, 0); }
+    __device__ __forceinline__ int32_t at(int j) const { return j == 0 ? lo16(a.x) : j == 1 ? hi16(a.x) : j == 2 ? lo16(a.y) : hi16(a.y); }
+};
 template <typename AccT> struct Acc4Of;
+template <> struct Acc4Of<int16_t> { using T = Acc4s; };
 template <> struct Acc4Of<int32_t> { using T = Acc4i; };
 template <> struct Acc4Of<int64_t> { using T = Acc4l; };
 
@@ -435,11 +470,11 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
             const int32_t r = __shfl_sync(FULL, start, u), l = __shfl_sync(FULL, len, u);
             AccT* acc = acc0 + __shfl_sync(FULL, to, u);
             if (8 * lane < l) {
-                Edges8<AccT> e;
+                Edges8<typename SumOf<AccT>::T> e;
                 e.load(N, (int64_t)(uint32_t)r + 8 * lane);
 #pragma unroll
                 for (int c = 0; c < 8; c++)
-                    if (e.w[c] != 0) red_add(acc + e.c[c], e.w[c]);
+                    if (e.w[c] != 0) red_acc(acc + e.c[c], e.w[c]);
             }
         }
     }
@@ -460,9 +495,17 @@ __device__ __noinline__ void advance_pairs(const PersistParams& P, int32_t quad,
     const uint32_t np = (uint32_t)N.n_pad, lp = (uint32_t)(first_pair(P) + (quad < 0 ? 0 : k));
     const int32_t bl = (int32_t)(lp / np), i = (int32_t)(lp - (uint32_t)bl * np);
     const bool on = quad >= 0 && i < N.n;
+    AccT* const acc = reinterpret_cast<AccT*>(S.acc) + (int64_t)P.b0 * np + lp;
+    const int64_t slot_stride = (int64_t)N.B * np;
+    typename SumOf<AccT>::T x[KB];
+#pragma unroll
+    for (int s = 0; s < KB; s++) {
+        const int sl = slot0 + s < S.n_slots ? slot0 + s : slot0 + s - S.n_slots;
+        x[s] = on && s < kc ? ld_acc(acc + sl * slot_stride) : 0;
+    }
     uint32_t* kw = smem_at<uint32_t>(P.lay.kick) + par * ((P.per + 3) / 4) + (quad < 0 ? 0 : quad);
     const uint32_t kick = on ? *kw >> j : 0u;
-    __syncwarp();
+    __syncwarp();                                               // (a quad's words are read before they are cleared)
     if (on && j == 0 && *kw != 0u) *kw = 0u;
     if (!on) return;
     float* sv = smem_at<float>(P.lay.v) + k;
@@ -472,14 +515,6 @@ __device__ __noinline__ void advance_pairs(const PersistParams& P, int32_t quad,
     const int na = smem_at<int32_t>(P.lay.ticks + 1024)[par * 64 + bl];
     const uint32_t f = *sr;
     const Lif<float> L = N.L32;
-    AccT* const acc = reinterpret_cast<AccT*>(S.acc) + (int64_t)P.b0 * np + lp;
-    const int64_t slot_stride = (int64_t)N.B * np;
-    AccT x[KB];
-#pragma unroll
-    for (int s = 0; s < KB; s++) {
-        const int sl = slot0 + s < S.n_slots ? slot0 + s : slot0 + s - S.n_slots;
-        x[s] = s < kc ? ld_cg(acc + sl * slot_stride) : 0;
-    }
     int64_t px[KB];
     int64_t* ring = nullptr;
     if (PLASTIC) {
@@ -497,7 +532,7 @@ __device__ __noinline__ void advance_pairs(const PersistParams& P, int32_t quad,
 #pragma unroll
     for (int s = 0; s < KB; s++) {
         const int sl = slot0 + s < S.n_slots ? slot0 + s : slot0 + s - S.n_slots;
-        if (x[s] != 0) acc[sl * slot_stride] = 0;
+        if (x[s] != 0) clear_acc(acc + sl * slot_stride);
         if (s < na) {
             float buf = acc_to_real<float>(x[s], L.w_syn);
             if (PLASTIC && ring) {
@@ -854,12 +889,13 @@ inline PersistPlan plan_persistent(int64_t n, int64_t n_pad, int32_t B, bool f64
     return P;
 }
 
-// Steps per epoch: 3K <= n_delay. The 2K accumulator slots of the group stay in L2 beside the
-// connectome's rows up to K = 4 at full scale; a smaller group runs longer epochs (fewer barriers).
+// Steps per epoch: 3K <= n_delay. Longer epochs mean fewer barriers, but the 2K accumulator slots of the
+// group are to stay in L2: in 16 bits K = 6 takes 53 MB for 16 whole brains (4.53 us per step, 4.80 with
+// K = 4); in 32 bits it takes 106 MB and was slower (7.9 us per step, 5.5 with K = 4).
 inline int persistent_epoch(const PersistPlan& P, int64_t n_pad, int n_delay, int acc_bytes)
 {
     const int64_t slot = (int64_t)P.group * n_pad * acc_bytes;
-    const int most = acc_bytes == 4 && slot * 2 * MAX_EPOCH <= (int64_t)48 << 20 ? MAX_EPOCH : 4;
+    const int most = acc_bytes == 2 && slot * 2 * MAX_EPOCH <= (int64_t)56 << 20 ? MAX_EPOCH : 4;
     return std::max(1, std::min(most, n_delay / 3));
 }
 
@@ -911,11 +947,12 @@ cudaError_t launch_persist_acc(const PersistPlan& P, const DevNet& N, const DevS
 }
 
 inline cudaError_t launch_persistent(const PersistPlan& P, const DevNet& N, const DevState& S, const PersistArgs& A,
-                                     int acc_mode, bool plastic, bool raster, bool record, cudaStream_t st)
+                                     int acc_bytes, bool plastic, bool raster, bool record, cudaStream_t st)
 {
-    if (acc_mode != 0) return launch_persist_acc<int64_t, 4>(P, N, S, A, plastic, raster, record, st);
-    if (A.epoch <= 4) return launch_persist_acc<int32_t, 4>(P, N, S, A, plastic, raster, record, st);
-    return launch_persist_acc<int32_t, MAX_EPOCH>(P, N, S, A, plastic, raster, record, st);
+    if (acc_bytes == 8) return launch_persist_acc<int64_t, 4>(P, N, S, A, plastic, raster, record, st);
+    if (acc_bytes == 4) return launch_persist_acc<int32_t, 4>(P, N, S, A, plastic, raster, record, st);
+    if (A.epoch <= 4) return launch_persist_acc<int16_t, 4>(P, N, S, A, plastic, raster, record, st);
+    return launch_persist_acc<int16_t, MAX_EPOCH>(P, N, S, A, plastic, raster, record, st);
 }
 
 }  // namespace fb

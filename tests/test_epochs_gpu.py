@@ -118,3 +118,40 @@ def test_engines_in_turn(torch):
         gb.set_schedule("step" if k % 2 else "persistent")
         _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps))
     gb.check()
+
+
+@pytest.mark.parametrize("top", [32_767, 32_768])
+def test_input_sums_at_the_edge_of_sixteen_bits(torch, top):
+    """Neighbouring neurons whose inputs of one step sum to +-top (every presynaptic neuron fires at once): the
+    16-bit accumulators hold 32,767, one more takes the 32-bit ones; partial resets and the step engine
+    in between."""
+    from flyzero_b200.brain import LIFParams
+    from flyzero_b200.gpu import BatchBrain
+
+    n, B, pre = 601, 3, 200
+    w = np.zeros((n, n), np.float32)
+    rng = np.random.default_rng(top)
+    for k, col in enumerate((400, 401, 402, 403, 599, 600)):
+        size = rng.multinomial(top - pre, np.full(pre, 1.0 / pre)) + 1
+        w[:pre, col] = size * (1 if k % 3 else -1)
+    w[:pre, 300:390] = rng.integers(-9, 9, (pre, 90))
+    gb = BatchBrain(sp.csr_matrix(w), LIFParams(), batch=B, seed=4)
+    eo = O.EngineOracle(sp.csr_matrix(w), O.Params(), batch=B, seed=4)
+    gb.set_schedule("persistent")
+    assert gb.info().epoch == (6 if top <= 32_767 else 4)
+    idx = np.arange(pre)
+    gb.set_input(idx, 20_000.0)                          # p > 1: every input neuron is kicked in every step
+    j = eo.slots(idx)
+    eo.p_ext[:, j] = np.float32(20_000.0) * np.float32(0.1 / 1000.0)
+    for k, steps in enumerate((20, 7, 30, 25, 3, 40)):
+        if k == 2:
+            gb.set_schedule("step")
+        if k == 3:
+            gb.reset([1])
+            eo.reset_flies([1])
+            gb.set_schedule("persistent")
+        if k == 4:
+            gb.reset([0, 2])
+            eo.reset_flies([0, 2])
+        _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps))
+    gb.check()
