@@ -51,6 +51,17 @@ class EyeParams(C.Structure):
                 ("transient_gain", C.c_double), ("sustained_gain", C.c_double), ("chromatic_gain", C.c_double)]
 
 
+class ColsumItem(C.Structure):
+    _fields_ = [("X", vp), ("grad", vp), ("N", C.c_int32), ("ld", C.c_int32)]
+
+
+class AdamItem(C.Structure):
+    _fields_ = [("w", vp), ("grad", vp), ("m", vp), ("v", vp), ("w_bf16", vp), ("w_bf16_t", vp), ("n", C.c_int64),
+                ("rows", C.c_int32), ("cols", C.c_int32), ("ldt", C.c_int32)]
+
+
+FS_LIST_MAX = 8
+
 _LIB = None
 
 # every symbol include/flybrain.h declares, with its signature
@@ -92,6 +103,8 @@ SIGNATURES = {
     "fs_colsum": (C.c_int, [vp, C.c_int32, C.c_int32, C.c_int32, vp, vp]),
     "fs_adam": (C.c_int, [vp, vp, vp, vp, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, vp, vp,
                           C.c_int32, C.c_int32, C.c_int32, vp]),
+    "fs_colsum_list": (C.c_int, [C.POINTER(ColsumItem), C.c_int32, C.c_int32, vp]),
+    "fs_adam_list": (C.c_int, [C.POINTER(AdamItem), C.c_int32, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, vp]),
     "fs_to_bf16": (C.c_int, [vp, C.c_int64, vp, vp, C.c_int32, C.c_int32, C.c_int32, vp]),
 }
 

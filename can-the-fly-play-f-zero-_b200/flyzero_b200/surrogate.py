@@ -130,6 +130,7 @@ class MLP:
         self._loss.zero_()
         _lib.check(self.L.fs_poisson_nll(_p(ws["Z"][-1]), _p(Y), M, d[-1], _p(self._loss), _p(ws["dZ"][-1]), OUT_PAD,
                                          _p(ws["dZT"][-1]), _stream(self.dev)))
+        sums = []
         for li in range(nl - 1, -1, -1):
             n, k = d[li + 1], d[li]
             A_in_T = ws["XTb"] if li == 0 else ws["HT"][li - 1]
@@ -137,26 +138,32 @@ class MLP:
             # dW = dZ^T X  (n x k): A = dZ^T (n x M), B = X^T (k x M)
             self._gemm(ws["dZT"][li], A_in_T, n, k, M, M, M, 0, out_f32=dW, ldo=k)
             ldz = OUT_PAD if li == nl - 1 else n
-            _lib.check(self.L.fs_colsum(_p(ws["dZ"][li]), M, n, ldz, _p(db), _stream(self.dev)))
+            sums.append(_lib.ColsumItem(ws["dZ"][li].data_ptr(), db.data_ptr(), n, ldz))
             if li > 0:
                 # dZ_prev = (dZ W) * gelu'(Z_prev): A = dZ (M x n), B = W^T (k x n)
                 self._gemm(ws["dZ"][li], self.WTb[li], M, k, n, ldz, self.WTb[li].shape[1], 3, zin=ws["Z"][li - 1],
                            out_bf16=ws["dZ"][li - 1], out_bf16_t=ws["dZT"][li - 1], ldo=k, ldo_t=M)
+        for at in range(0, nl, _lib.FS_LIST_MAX):
+            part = sums[at:at + _lib.FS_LIST_MAX]
+            _lib.check(self.L.fs_colsum_list((_lib.ColsumItem * len(part))(*part), len(part), M, _stream(self.dev)))
         return self._loss / M
 
     def step(self):
         """One Adam update from self.grads (then the bf16 copies follow)."""
         self.t += 1
         b1, b2 = self.betas
+        items = []
         for li in range(len(self.W)):
             W, b = self.W[li], self.b[li]
-            gW, gb = self.grads[li]
+            (gW, gb), (mW, mb), (vW, vb) = self.grads[li], self.m[li], self.v[li]
             n, k = W.shape
-            _lib.check(self.L.fs_adam(_p(W), _p(gW), _p(self.m[li][0]), _p(self.v[li][0]), W.numel(), self.lr, b1, b2,
-                                      self.eps, self.t, _p(self.Wb[li]), _p(self.WTb[li]), n, k, self.WTb[li].shape[1],
-                                      _stream(self.dev)))
-            _lib.check(self.L.fs_adam(_p(b), _p(gb), _p(self.m[li][1]), _p(self.v[li][1]), b.numel(), self.lr, b1, b2,
-                                      self.eps, self.t, None, None, 0, 0, 0, _stream(self.dev)))
+            items.append(_lib.AdamItem(W.data_ptr(), gW.data_ptr(), mW.data_ptr(), vW.data_ptr(), self.Wb[li].data_ptr(),
+                                       self.WTb[li].data_ptr(), W.numel(), n, k, self.WTb[li].shape[1]))
+            items.append(_lib.AdamItem(b.data_ptr(), gb.data_ptr(), mb.data_ptr(), vb.data_ptr(), None, None, b.numel(), 0, 0, 0))
+        for at in range(0, len(items), _lib.FS_LIST_MAX):
+            part = items[at:at + _lib.FS_LIST_MAX]
+            _lib.check(self.L.fs_adam_list((_lib.AdamItem * len(part))(*part), len(part), self.lr, b1, b2, self.eps, self.t,
+                                           _stream(self.dev)))
 
     def train_step(self, X, Y):
         self.forward(X, training=True)

@@ -61,12 +61,35 @@ int fs_poisson_nll(const float* z, const float* y, int32_t M, int32_t D, double*
 /* Column sums of a bf16 matrix (M x N, row stride ld) into FP32 grad[N] (the bias gradient). */
 int fs_colsum(const uint16_t* X, int32_t M, int32_t N, int32_t ld, float* grad, void* stream);
 
+/* The column sums of up to FS_LIST_MAX matrices of M rows in one launch. */
+#define FS_LIST_MAX 8
+typedef struct fs_colsum_item {
+    const uint16_t* X;
+    float* grad;
+    int32_t N, ld;
+} fs_colsum_item;
+int fs_colsum_list(const fs_colsum_item* items /*[host]*/, int32_t count, int32_t M, void* stream);
+
 /* Adam on FP32 master weights w[n] with FP32 moments m, v: bias-corrected with step t (>= 1);
  * writes the bf16 copy w_bf16 (same layout) and, when w_bf16_t != NULL, the transposed bf16 copy
  * of the rows x cols weight (rows * cols == n, 0 < rows <= 2,097,120) with row stride ldt >= rows. */
 int fs_adam(float* w, const float* grad, float* m, float* v, int64_t n, float lr, float beta1, float beta2,
             float eps, int32_t t, uint16_t* w_bf16, uint16_t* w_bf16_t, int32_t rows, int32_t cols, int32_t ldt,
             void* stream);
+
+/* The same update of up to FS_LIST_MAX parameters in one launch (fields as fs_adam's arguments). */
+typedef struct fs_adam_item {
+    float* w;
+    const float* grad;
+    float* m;
+    float* v;
+    uint16_t* w_bf16;
+    uint16_t* w_bf16_t;
+    int64_t n;
+    int32_t rows, cols, ldt;
+} fs_adam_item;
+int fs_adam_list(const fs_adam_item* items /*[host]*/, int32_t count, float lr, float beta1, float beta2, float eps,
+                 int32_t t, void* stream);
 
 /* FP32 -> bf16 (round to nearest even); optional transposed copy of the rows x cols matrix
  * (rows * cols == n, 0 < rows <= 2,097,120) with row stride ldt >= rows. */
