@@ -107,7 +107,22 @@ class BatchMotor:
         _lib.check(b._L.fb_group_rates(b._h, _p(counts), _p(self.g.idx), _p(self.g.ptr), self.g.n_groups, _p(self.w),
                                        float(a), float(hz), _p(self.rates_dev), _stream(b.device)))
         rates = self.rates
-        return [self.buttons(r, k) for k, r in enumerate(rates)]
+        if type(self).buttons is not BatchMotor.buttons or self.p.taps:
+            return [self.buttons(r, k) for k, r in enumerate(rates)]
+        return self._all_buttons(rates)
+
+    def _all_buttons(self, r) -> list:
+        """``buttons`` of every slot at once (without taps): the same float32 comparisons on columns, a dict per
+        slot from the results (slot by slot the scalars took 150 of a 230 us update of 64 slots)."""
+        p = self.p
+        steer = (r[:, 0] - r[:, 1]) + (r[:, 5] - r[:, 4]) + p.steer_bias
+        lean = r[:, 2] - r[:, 3]
+        on = [(steer > p.steer_threshold), (steer < -p.steer_threshold), (lean > p.lean_threshold),
+              (lean < -p.lean_threshold), (r[:, 6] > p.accel_threshold), (r[:, 7] > p.brake_threshold),
+              (r[:, 8] > p.boost_threshold)]
+        return [{"B": acc, "Y": brake, "A": boost, "X": False, "L": lean_l, "R": lean_r, "LEFT": left, "RIGHT": right,
+                 "UP": False, "DOWN": False, "SELECT": False, "START": False}
+                for left, right, lean_l, lean_r, acc, brake, boost in zip(*(c.tolist() for c in on))]
 
     def _tap(self, k, j, x, threshold, span):
         """Pulse-density modulation of a steering command: a first-order sigma-delta quantiser.
