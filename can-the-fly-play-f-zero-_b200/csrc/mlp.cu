@@ -27,6 +27,20 @@ namespace {
 
 constexpr int BM = 128, BN = 64, BK = 32, PADK = BK + 8;
 
+// Programmatic dependent launch: the surrogate's kernels form a chain of launches of a few microseconds, each
+// the next one's only predecessor. A kernel lets its successor be set up while it runs (at its start) and
+// itself waits, before it touches any global memory, until its predecessor has completed and its
+// writes are visible. Every block executes both before its first return, so completion stays transitive
+// along the stream, and a block waits only for blocks that are already resident (with their TMEM): a
+// successor starts when all of its predecessor's blocks have come this far. Between ordinary launches
+// the drain, launch and set-up of the next kernel were 1-2 us of every 4: a training step at batch 2048
+// goes from 158 to 134 us with the chain, a screen of 512 inputs from 41.8 to 33.6 us.
+__device__ __forceinline__ void pdl_chain()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ uint16_t f2bf(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
@@ -474,6 +488,7 @@ __global__ void __launch_bounds__(TMA_THREADS) k_gemm_tma(const __grid_constant_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    pdl_chain();                                      // (barriers and TMEM are set up beside the predecessor)
     const uint32_t tmem = s_tmem;
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
     // this block's K tiles: all of them, or its share of a split (every share has at least one)
@@ -620,6 +635,7 @@ __global__ void __launch_bounds__(TMA_THREADS) k_gemm_tma(const __grid_constant_
 
 __global__ void k_poisson(const float* z, const float* y, int M, int D, double* loss, uint16_t* dz, int ldd, uint16_t* dz_t)
 {
+    pdl_chain();
     __shared__ double part[8];
     double s = 0.0;
     const int64_t total = (int64_t)M * D;
@@ -652,6 +668,7 @@ struct ColsumList {
 };
 __global__ void __launch_bounds__(1024) k_colsum(const ColsumList L)
 {
+    pdl_chain();
     __shared__ float part[32][33];
     __shared__ float tot[32];
     int which = 0;
@@ -706,6 +723,7 @@ struct AdamList {
 };
 __global__ void __launch_bounds__(256) k_adam(const AdamList A, float lr, float b1, float b2, float eps, float c1, float c2)
 {
+    pdl_chain();
     __shared__ uint16_t tile[32][34];
     int which = 0;
 #pragma unroll
@@ -749,6 +767,7 @@ __global__ void __launch_bounds__(256) k_adam(const AdamList A, float lr, float 
 
 __global__ void k_to_bf16(const float* x, int64_t n, uint16_t* out)
 {
+    pdl_chain();
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x)
         out[p] = f2bf(x[p]);
 }
@@ -757,6 +776,7 @@ __global__ void k_to_bf16(const float* x, int64_t n, uint16_t* out)
 // and the transposed one, both stored along rows
 __global__ void k_to_bf16_t(const float* x, uint16_t* out, uint16_t* out_t, int rows, int cols, int ldt)
 {
+    pdl_chain();
     __shared__ uint16_t tile[32][34];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, tx = threadIdx.x, ty = threadIdx.y;
     for (int k = ty; k < 32; k += 8) {
@@ -779,6 +799,7 @@ __global__ void k_to_bf16_t(const float* x, uint16_t* out, uint16_t* out_t, int 
 // multiples of 4, every base aligned): 4096 x 1280 in 9 us, element by element 18.6. Bound by memory.
 __global__ void __launch_bounds__(256) k_to_bf16_t4(const float* x, uint16_t* out, uint16_t* out_t, int rows, int cols, int ldt)
 {
+    pdl_chain();
     __shared__ uint16_t tile[64][64 + 4];              // [column][row]
     const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64, lane = threadIdx.x & 15, w = threadIdx.x >> 4;
     float4 q[4];
@@ -825,6 +846,27 @@ int cuda_status()
     if (e == cudaSuccess) return FB_OK;
     fb::set_last_error(cudaGetErrorString(e));
     return FB_ERR_CUDA;
+}
+
+// A launch of the chain (pdl_chain), as clusters of 1 x cy x cz blocks
+template <typename... P, typename... A>
+cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cy, unsigned cz, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 1;
+    at[1].val.clusterDim.y = cy;
+    at[1].val.clusterDim.z = cz;
+    cfg.attrs = at;
+    cfg.numAttrs = cy * cz > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 template <int BN>
@@ -899,23 +941,9 @@ int launch_tma(const uint16_t* A, const uint16_t* B, int M, int N, int K, int ld
     }
     const unsigned gx = (N + BN - 1) / BN, gy = (M + TC_BM - 1) / TC_BM;
     const int S = split_for((int)(gx * gy), K, smem * 2 <= 227 * 1024 ? 2 : 1);
-    if (S == 1) {
-        k_gemm_tma<BN><<<dim3(gx, gy), TMA_THREADS, smem, st>>>(ma, mb, M, N, K, e);
-    } else {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(gx, gy, (unsigned)S);
-        cfg.blockDim = dim3(TMA_THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 1;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = (unsigned)S;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, k_gemm_tma<BN>, ma, mb, M, N, K, e) != cudaSuccess) return -cuda_status();
-    }
+    if (launch_chain(k_gemm_tma<BN>, dim3(gx, gy, (unsigned)S), dim3(TMA_THREADS), smem, st, 1u, (unsigned)S, ma, mb, M, N, K, e) !=
+        cudaSuccess)
+        return -cuda_status();
     const int rc = cuda_status();
     return rc == FB_OK ? 1 : -rc;
 }
@@ -972,7 +1000,7 @@ extern "C" int fs_poisson_nll(const float* z, const float* y, int32_t M, int32_t
                               int32_t ldd, uint16_t* dz_t, void* stream)
 {
     if (!z || !y || !loss_sum || !dz || M <= 0 || D <= 0 || ldd < D) return fail("fs_poisson_nll: bad arguments");
-    k_poisson<<<blocks_for((int64_t)M * D), 256, 0, (cudaStream_t)stream>>>(z, y, M, D, loss_sum, dz, ldd, dz_t);
+    launch_chain(k_poisson, blocks_for((int64_t)M * D), 256, 0, (cudaStream_t)stream, 1, 1, z, y, M, D, loss_sum, dz, ldd, dz_t);
     return cuda_status();
 }
 
@@ -990,22 +1018,7 @@ extern "C" int fs_colsum_list(const fs_colsum_item* items, int32_t count, int32_
         blocks += (it.N + 31) / 32;
     }
     const int S = std::min(MAX_SPLIT, std::max(1, M / 256));    // >= 8 rows per warp
-    if (S == 1) {
-        k_colsum<<<blocks, 1024, 0, (cudaStream_t)stream>>>(L);
-        return cuda_status();
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks, (unsigned)S);
-    cfg.blockDim = dim3(1024);
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 1;
-    at[0].val.clusterDim.y = (unsigned)S;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_colsum, L) != cudaSuccess) return cuda_status();
+    launch_chain(k_colsum, dim3((unsigned)blocks, (unsigned)S), dim3(1024), 0, (cudaStream_t)stream, (unsigned)S, 1, L);
     return cuda_status();
 }
 
@@ -1040,7 +1053,7 @@ extern "C" int fs_adam_list(const fs_adam_item* items, int32_t count, float lr, 
         if (blocks > INT32_MAX) return fail("fs_adam: too many elements");
     }
     const float c1 = 1.0f - powf(beta1, (float)t), c2 = 1.0f - powf(beta2, (float)t);
-    k_adam<<<(unsigned)blocks, dim3(32, 8), 0, (cudaStream_t)stream>>>(A, lr, beta1, beta2, eps, c1, c2);
+    launch_chain(k_adam, dim3((unsigned)blocks), dim3(32, 8), 0, (cudaStream_t)stream, 1, 1, A, lr, beta1, beta2, eps, c1, c2);
     return cuda_status();
 }
 
@@ -1060,12 +1073,12 @@ extern "C" int fs_to_bf16(const float* x, int64_t n, uint16_t* out, uint16_t* ou
         return fail("fs_to_bf16: the transposed copy needs 0 < rows <= 2097120, rows * cols == n and ldt >= rows");
     if (out_t && cols % 4 == 0 && ldt % 4 == 0 && (((uintptr_t)x & 15) | ((uintptr_t)out & 7) | ((uintptr_t)out_t & 7)) == 0) {
         const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64));
-        k_to_bf16_t4<<<grid, 256, 0, (cudaStream_t)stream>>>(x, out, out_t, rows, cols, ldt);
+        launch_chain(k_to_bf16_t4, grid, dim3(256), 0, (cudaStream_t)stream, 1, 1, x, out, out_t, rows, cols, ldt);
     } else if (out_t) {
         const dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
-        k_to_bf16_t<<<grid, dim3(32, 8), 0, (cudaStream_t)stream>>>(x, out, out_t, rows, cols, ldt);
+        launch_chain(k_to_bf16_t, grid, dim3(32, 8), 0, (cudaStream_t)stream, 1, 1, x, out, out_t, rows, cols, ldt);
     } else {
-        k_to_bf16<<<blocks_for(n), 256, 0, (cudaStream_t)stream>>>(x, n, out);
+        launch_chain(k_to_bf16, blocks_for(n), 256, 0, (cudaStream_t)stream, 1, 1, x, n, out);
     }
     return cuda_status();
 }
