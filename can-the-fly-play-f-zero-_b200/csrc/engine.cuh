@@ -26,6 +26,7 @@
 // order-free, so this equals the reference's push-at-spike-time ring (brain.py:54-56) exactly.
 // Plastic weights may change between runs, so their rows are pushed at spike time.
 #pragma once
+#include "chain.cuh"
 #include "common.cuh"
 
 namespace fb {
@@ -241,70 +242,56 @@ __device__ __forceinline__ bool kick_of(const DevState& S, const uint32_t* kicks
     return p > 0.0f && hash_kick(tid, step_no, S.seed, (uint32_t)b, p);
 }
 
-// ---------------------------------------------------------------------------------------------
-// Step engine, kernel 1: every (instance, neuron) advances one step; spikes become work items.
-// ---------------------------------------------------------------------------------------------
+// Step engine, one part: the pairs (b, i) of a warp advance one step; spikes become work items.
 template <typename Real, typename AccT, bool RASTER, bool PLASTIC, bool RECORD>
-__global__ void __launch_bounds__(256) k_update(const DevNet N, const DevState S, const StepArgs A)
+__device__ __forceinline__ void update_pair(const DevNet& N, const DevState& S, const StepArgs& A, int32_t b, int64_t i64)
 {
-    const int64_t n = N.n;
-    const int64_t total = (int64_t)N.B * n;
+    const int64_t n = N.n, t = A.t;
     const Lif<Real>& L = lif_of<Real>(N);
-    const int64_t t = A.t;
-    if (blockIdx.x == 0)       // the lists consumed by the push at t-1 start empty again
-        for (int32_t k = threadIdx.x; k < S.n_groups; k += blockDim.x) *count_of(S, pos_mod(t - N.n_delay, N.R), k) = 0;
-    AccT* acc = acc_slot<AccT>(N, S, t);
-    Real* V = reinterpret_cast<Real*>(S.v);
-    Real* G = reinterpret_cast<Real*>(S.g);
     const int64_t slot = pos_mod(t, N.R);
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < total; base += stride) {
-        const int64_t pair = base + threadIdx.x;
-        int nch = 0;
-        int32_t b = 0, i = 0;
-        if (pair < total) {
-            b = (int32_t)(pair / n);
-            i = (int32_t)(pair - (int64_t)b * n);
-            if (t < S.stop_tick[b]) {
-                AccT* ap = acc + (int64_t)b * N.n_pad + i;
-                const AccT x = *ap;
-                if (x != 0) *ap = 0;
-                Real buf = acc_to_real<Real>(x, L.w_syn);
-                if (PLASTIC && N.ppost_of[i] >= 0) buf = add_rn(buf, take_plastic<Real>(N, S, t, b, i));
-                Real v = V[pair], g = G[pair];
-                const Real v0 = v, g0 = g;
-                const int r0 = S.ref[pair];
-                int r = r0;
-                const int32_t j = S.ext_idx[i];
-                float bias = 0.0f;
-                bool kicked = false;
-                if (j >= 0) {
-                    bias = S.bias_ext[(int64_t)b * S.n_ext + j];
-                    kicked = kick_of<RASTER>(S, A.kicks, A.words, N.B, A.s, b, j, (uint32_t)pair, A.step_no);
-                }
-                // the engine always fuses the two multiply-adds, as the shipped reference kernel does
-                const bool spk = lif_step<Real>(v, g, r, buf, j >= 0, bias, kicked, L, N.n_ref, true);
-                if (bits_differ(g, g0)) G[pair] = g;
-                if (bits_differ(v, v0)) V[pair] = v;
-                if (r != r0) S.ref[pair] = (int8_t)r;
-                if (spk) {
-                    A.counts[pair] += 1;
-                    if (S.masks)
-                        atomicOr(S.masks + (slot * n + i) * S.mask_words + (b >> 6), 1ull << (b & 63));
-                    const int64_t len = N.rowptr[i + 1] - N.rowptr[i];
-                    nch = (int)((len + CHUNK - 1) / CHUNK);
-                    if (PLASTIC) push_plastic_row(N, S, t, b, i);
-                    if (RECORD) {
-                        if (A.step_counts) atomicAdd(A.step_counts + (int64_t)A.s * N.B + b, 1);
-                        if (A.step_digest)
-                            atomicAdd(reinterpret_cast<unsigned long long*>(A.step_digest + (int64_t)A.s * N.B + b),
-                                      (unsigned long long)spike_tag((uint64_t)i));
-                    }
-                }
+    const int32_t i = (int32_t)i64;
+    int nch = 0;
+    if (i64 < n && t < S.stop_tick[b]) {
+        const int64_t pair = (int64_t)b * n + i;
+        AccT* ap = acc_slot<AccT>(N, S, t) + (int64_t)b * N.n_pad + i;
+        Real* pv = reinterpret_cast<Real*>(S.v) + pair;
+        Real* pg = reinterpret_cast<Real*>(S.g) + pair;
+        const AccT x = *ap;                              // (independent loads: in flight together)
+        Real v = *pv, g = *pg;
+        const int r0 = S.ref[pair];
+        const int32_t j = S.ext_idx[i];
+        const bool target = PLASTIC && N.ppost_of[i] >= 0;
+        if (x != 0) *ap = 0;
+        Real buf = acc_to_real<Real>(x, L.w_syn);
+        if (target) buf = add_rn(buf, take_plastic<Real>(N, S, t, b, i));
+        const Real v0 = v, g0 = g;
+        int r = r0;
+        float bias = 0.0f;
+        bool kicked = false;
+        if (j >= 0) {
+            bias = S.bias_ext[(int64_t)b * S.n_ext + j];
+            kicked = kick_of<RASTER>(S, A.kicks, A.words, N.B, A.s, b, j, (uint32_t)pair, A.step_no);
+        }
+        // the engine always fuses the two multiply-adds, as the shipped reference kernel does
+        const bool spk = lif_step<Real>(v, g, r, buf, j >= 0, bias, kicked, L, N.n_ref, true);
+        if (bits_differ(g, g0)) *pg = g;
+        if (bits_differ(v, v0)) *pv = v;
+        if (r != r0) S.ref[pair] = (int8_t)r;
+        if (spk) {
+            A.counts[pair] += 1;
+            if (S.masks) atomicOr(S.masks + (slot * n + i) * S.mask_words + (b >> 6), 1ull << (b & 63));
+            const int64_t len = N.rowptr[i + 1] - N.rowptr[i];
+            nch = (int)((len + CHUNK - 1) / CHUNK);
+            if (PLASTIC) push_plastic_row(N, S, t, b, i);
+            if (RECORD) {
+                if (A.step_counts) atomicAdd(A.step_counts + (int64_t)A.s * N.B + b, 1);
+                if (A.step_digest)
+                    atomicAdd(reinterpret_cast<unsigned long long*>(A.step_digest + (int64_t)A.s * N.B + b),
+                              (unsigned long long)spike_tag((uint64_t)i));
             }
         }
-        warp_append(N, S, slot, nch, i, b);
     }
+    warp_append(N, S, slot, nch, i, b);
 }
 
 // 8 consecutive CSR entries of one lane: weights (one or four 16-byte loads) and columns (two).
@@ -385,28 +372,22 @@ __device__ __forceinline__ void push_range(const DevNet& N, const DevState& S, i
     }
 }
 
-// ---------------------------------------------------------------------------------------------
-// Step engine, kernel 2: the spikes of step t+1-n_delay (they arrive at step t+1) are scattered
-// into the accumulator that step t+1 reads; each block takes a contiguous share of every list.
-// ---------------------------------------------------------------------------------------------
 // The spike-mask slot that step t+1 records into starts empty (it last held step t-n_delay, whose
 // propagation ran at step t-1).
-__device__ __forceinline__ void clear_mask_slot(const DevNet& N, const DevState& S, int64_t t)
+__device__ __forceinline__ void clear_mask_slot(const DevNet& N, const DevState& S, int64_t t, int blk, int n_blk)
 {
     if (!S.masks) return;
     const int64_t words = N.n * S.mask_words;
     unsigned long long* m = S.masks + pos_mod(t + 1, N.R) * words;
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < words; k += (int64_t)gridDim.x * blockDim.x)
-        m[k] = 0ull;
+    for (int64_t k = (int64_t)blk * blockDim.x + threadIdx.x; k < words; k += (int64_t)n_blk * blockDim.x) m[k] = 0ull;
 }
 
-// `do_push` 0: the arrivals of t+1 were pushed ahead already (by the persistent engine); only the
-// mask slot is cleared.
-template <typename AccT, int LANES>
-__global__ void __launch_bounds__(256) k_push(const DevNet N, const DevState S, int64_t t, int do_push)
+// Step engine, the other part, block `blk` of `n_blk`: the spikes of step t+1-n_delay (they arrive at
+// step t+1) are scattered into the accumulator that step t+1 reads; each block takes a contiguous
+// share of every list.
+template <typename AccT>
+__device__ __forceinline__ void push_lists(const DevNet& N, const DevState& S, int64_t t, int lanes, int blk, int n_blk)
 {
-    clear_mask_slot(N, S, t);
-    if (!do_push || t + 1 - N.n_delay < 0) return;
     AccT* acc = acc_slot<AccT>(N, S, t + 1);
     const int64_t slot = pos_mod(t + 1 - N.n_delay, N.R);
     __shared__ int32_t s_total;
@@ -414,14 +395,50 @@ __global__ void __launch_bounds__(256) k_push(const DevNet N, const DevState S, 
         if (threadIdx.x == 0) s_total = list_length(S, slot, q);     // (one load per block: they all hit one address)
         __syncthreads();
         const int64_t total = s_total;
-        const int64_t g0 = total * blockIdx.x / gridDim.x, g1 = total * (blockIdx.x + 1) / gridDim.x;
-        push_range<AccT, LANES>(N, S, t, q, acc, g0, g1, threadIdx.x / LANES, blockDim.x / LANES, threadIdx.x % LANES);
+        const int64_t g0 = total * blk / n_blk, g1 = total * (blk + 1) / n_blk;
+        const int64_t lg = threadIdx.x / lanes, n_lg = blockDim.x / lanes;
+        const int lane = threadIdx.x % lanes;
+        if (lanes == 8) push_range<AccT, 8>(N, S, t, q, acc, g0, g1, lg, n_lg, lane);
+        else if (lanes == 16) push_range<AccT, 16>(N, S, t, q, acc, g0, g1, lg, n_lg, lane);
+        else push_range<AccT, 32>(N, S, t, q, acc, g0, g1, lg, n_lg, lane);
         __syncthreads();
     }
 }
 
 // ---------------------------------------------------------------------------------------------
-// Pull propagation (step engine, kernel 2 alternative): every postsynaptic neuron j gathers its
+// Step engine: one launch per step. The first n_push blocks scatter the spikes that arrive at t+1, the
+// others advance every (instance, neuron) through step t, `per` blocks an instance. The two touch
+// different accumulator slots (t+1 and t) and, with n_delay >= 2, different lists: the pushed one
+// (step t+1-n_delay) was filled by an earlier launch, the one that starts empty here held step t-n_delay,
+// pushed by the launch before. With n_delay = 1 the pushed spikes are this step's own, so the host
+// launches the two parts one after the other (n_push = 0, then pushing blocks alone).
+// `do_push` 0: the arrivals of t+1 were pushed ahead already (by the persistent engine); only the mask
+// slot is cleared.
+// ---------------------------------------------------------------------------------------------
+struct StepGrid {
+    int32_t n_push, per;       // pushing blocks; updating blocks per instance
+    int32_t do_push, lanes;
+};
+
+template <typename Real, typename AccT, bool RASTER, bool PLASTIC, bool RECORD>
+__global__ void __launch_bounds__(256) k_step(const __grid_constant__ DevNet N, const __grid_constant__ DevState S,
+                                              const __grid_constant__ StepArgs A, const StepGrid G)
+{
+    pdl_chain();
+    if ((int)blockIdx.x < G.n_push) {
+        clear_mask_slot(N, S, A.t, (int)blockIdx.x, G.n_push);
+        if (G.do_push && A.t + 1 - N.n_delay >= 0) push_lists<AccT>(N, S, A.t, G.lanes, (int)blockIdx.x, G.n_push);
+        return;
+    }
+    const uint32_t u = blockIdx.x - (uint32_t)G.n_push;
+    const int32_t b = (int32_t)(u / (uint32_t)G.per);
+    if (u == 0)                // the lists consumed by the push at t-1 start empty again
+        for (int32_t k = threadIdx.x; k < S.n_groups; k += blockDim.x) *count_of(S, pos_mod(A.t - N.n_delay, N.R), k) = 0;
+    update_pair<Real, AccT, RASTER, PLASTIC, RECORD>(N, S, A, b, (int64_t)(u % (uint32_t)G.per) * blockDim.x + threadIdx.x);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Pull propagation (step engine, in place of the pushing blocks): every postsynaptic neuron j gathers its
 // incoming entries whose presynaptic neuron spiked at step s = t+1-n_delay, for the instances of
 // one 64-bit mask word per thread. The sums are exact integers, so push and pull give identical
 // accumulators; pull reads the whole connectome once per step for all instances, push only the
@@ -434,7 +451,7 @@ template <> __device__ __forceinline__ int64_t pull_weight<int64_t>(const DevNet
 template <typename AccT>
 __global__ void __launch_bounds__(256) k_pull(const DevNet N, const DevState S, int64_t t)
 {
-    clear_mask_slot(N, S, t);
+    clear_mask_slot(N, S, t, (int)blockIdx.x, (int)gridDim.x);
     const int64_t s = t + 1 - N.n_delay;
     if (s < 0) return;
     AccT* acc = acc_slot<AccT>(N, S, t + 1);

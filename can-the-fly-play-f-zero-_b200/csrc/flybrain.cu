@@ -374,9 +374,6 @@ int largest_input(fb_brain* h, int64_t* out)
     return FB_OK;
 }
 
-int dispatch_step(fb_brain* h, const StepArgs& A, bool raster, bool record, cudaStream_t st);
-int dispatch_push(fb_brain* h, int64_t t, cudaStream_t st);
-int dispatch_pull(fb_brain* h, int64_t t, cudaStream_t st);
 
 // Build what pull propagation needs: the connectome by postsynaptic neuron and the spike-mask
 // ring (zeroed; masks are recorded from the current step on). The device must be idle.
@@ -910,11 +907,12 @@ extern "C" int fb_check(fb_brain* h, void* stream)
 namespace {
 
 template <typename Real, typename AccT>
-void launch_update(fb_brain* h, const StepArgs& A, bool raster, bool plastic, bool record, int blocks, cudaStream_t st)
+void launch_step(fb_brain* h, const StepArgs& A, const StepGrid& G, bool raster, bool plastic, bool record, unsigned blocks,
+                 cudaStream_t st)
 {
     const DevNet N = h->net();
     const DevState S = h->state();
-#define L_(R_, P_, C_) k_update<Real, AccT, R_, P_, C_><<<blocks, 256, 0, st>>>(N, S, A)
+#define L_(R_, P_, C_) launch_chain(k_step<Real, AccT, R_, P_, C_>, blocks, 256, 0, st, 1, 1, N, S, A, G)
     if (raster) {
         if (plastic) { if (record) L_(true, true, true); else L_(true, true, false); }
         else { if (record) L_(true, false, true); else L_(true, false, false); }
@@ -925,30 +923,26 @@ void launch_update(fb_brain* h, const StepArgs& A, bool raster, bool plastic, bo
 #undef L_
 }
 
-int dispatch_step(fb_brain* h, const StepArgs& A, bool raster, bool record, cudaStream_t st)
+// One launch of the step engine: the updating blocks, the pushing blocks, or both
+int dispatch_step(fb_brain* h, const StepArgs& A, bool update, bool push, bool raster, bool record, cudaStream_t st)
 {
-    const int64_t total = (int64_t)h->B * h->n;
-    const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)h->sm_count * 16);
+    StepGrid G{};
+    G.per = (int32_t)((h->n + 255) / 256);
+    G.n_push = push ? (int32_t)std::min<int64_t>(std::max<int64_t>(h->sm_count, (int64_t)h->B * 16), (int64_t)h->sm_count * 8) : 0;
+    G.do_push = A.t + 1 >= h->pushed_until;            // else pushed ahead by the persistent engine
+    G.lanes = h->lanes;
+    const unsigned blocks = (unsigned)G.n_push + (update ? (unsigned)G.per * (unsigned)h->B : 0u);
     const bool plastic = h->n_pl > 0;
     if (h->f64) {
-        if (h->acc_mode == 0) launch_update<double, int32_t>(h, A, raster, plastic, record, blocks, st);
-        else launch_update<double, int64_t>(h, A, raster, plastic, record, blocks, st);
+        if (h->acc_mode == 0) launch_step<double, int32_t>(h, A, G, raster, plastic, record, blocks, st);
+        else launch_step<double, int64_t>(h, A, G, raster, plastic, record, blocks, st);
     } else {
-        if (h->acc_mode == 0) launch_update<float, int32_t>(h, A, raster, plastic, record, blocks, st);
-        else launch_update<float, int64_t>(h, A, raster, plastic, record, blocks, st);
+        if (h->acc_mode == 0) launch_step<float, int32_t>(h, A, G, raster, plastic, record, blocks, st);
+        else launch_step<float, int64_t>(h, A, G, raster, plastic, record, blocks, st);
     }
     CU(cudaGetLastError());
     h->launches += 1;
     return FB_OK;
-}
-
-template <typename AccT> void launch_push(fb_brain* h, int64_t t, int do_push, int blocks, cudaStream_t st)
-{
-    const DevNet N = h->net();
-    const DevState S = h->state();
-    if (h->lanes == 8) k_push<AccT, 8><<<blocks, 256, 0, st>>>(N, S, t, do_push);
-    else if (h->lanes == 16) k_push<AccT, 16><<<blocks, 256, 0, st>>>(N, S, t, do_push);
-    else k_push<AccT, 32><<<blocks, 256, 0, st>>>(N, S, t, do_push);
 }
 
 int dispatch_pull(fb_brain* h, int64_t t, cudaStream_t st)
@@ -959,17 +953,6 @@ int dispatch_pull(fb_brain* h, int64_t t, cudaStream_t st)
     const DevState S = h->state();
     if (h->acc_mode == 0) k_pull<int32_t><<<blocks, 256, 0, st>>>(N, S, t);
     else k_pull<int64_t><<<blocks, 256, 0, st>>>(N, S, t);
-    CU(cudaGetLastError());
-    h->launches += 1;
-    return FB_OK;
-}
-
-int dispatch_push(fb_brain* h, int64_t t, cudaStream_t st)
-{
-    const int blocks = (int)std::min<int64_t>(std::max<int64_t>(h->sm_count, (int64_t)h->B * 16), (int64_t)h->sm_count * 8);
-    const int do_push = t + 1 >= h->pushed_until;      // else pushed ahead by the persistent engine
-    if (h->acc_mode == 0) launch_push<int32_t>(h, t, do_push, blocks, st);
-    else launch_push<int64_t>(h, t, do_push, blocks, st);
     CU(cudaGetLastError());
     h->launches += 1;
     return FB_OK;
@@ -1029,12 +1012,13 @@ extern "C" int fb_run(fb_brain* h, int32_t steps, int32_t* counts_out, const uin
             StepArgs A{};
             A.t = h->t + s; A.step_no = h->step_no + (uint32_t)s; A.s = s; A.kicks = kicks; A.words = words;
             A.counts = counts_out; A.step_counts = step_counts; A.step_digest = step_digest;
-            int rc = dispatch_step(h, A, kicks != nullptr, record, st);
-            if (rc) return rc;
             // pull only for spike steps whose masks were recorded (else the work items serve)
             const bool pull = h->prop == FB_PROP_PULL && h->masks && A.t + 1 - h->n_delay >= h->mask_from &&
                               A.t + 1 >= h->pushed_until;
-            rc = pull ? dispatch_pull(h, A.t, st) : dispatch_push(h, A.t, st);
+            const bool together = !pull && h->n_delay >= 2;   // (the spikes of this very step are not pushed yet)
+            int rc = dispatch_step(h, A, true, together, kicks != nullptr, record, st);
+            if (!rc && pull) rc = dispatch_pull(h, A.t, st);
+            else if (!rc && !together) rc = dispatch_step(h, A, false, true, kicks != nullptr, record, st);
             if (rc) return rc;
             h->pushed_until = std::max<int64_t>(h->pushed_until, A.t + 2);
         }

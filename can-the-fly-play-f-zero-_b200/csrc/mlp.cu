@@ -18,6 +18,7 @@
 
 #include "../../include/flybrain.h"
 #include "../../include/flysurrogate.h"
+#include "chain.cuh"
 
 namespace fb {
 void set_last_error(const char* msg);
@@ -27,19 +28,11 @@ namespace {
 
 constexpr int BM = 128, BN = 64, BK = 32, PADK = BK + 8;
 
-// Programmatic dependent launch: the surrogate's kernels form a chain of launches of a few microseconds, each
-// the next one's only predecessor. A kernel lets its successor be set up while it runs (at its start) and
-// itself waits, before it touches any global memory, until its predecessor has completed and its
-// writes are visible. Every block executes both before its first return, so completion stays transitive
-// along the stream, and a block waits only for blocks that are already resident (with their TMEM): a
-// successor starts when all of its predecessor's blocks have come this far. Between ordinary launches
-// the drain, launch and set-up of the next kernel were 1-2 us of every 4: a training step at batch 2048
-// goes from 158 to 134 us with the chain, a screen of 512 inputs from 41.8 to 33.6 us.
-__device__ __forceinline__ void pdl_chain()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// The surrogate's kernels are launched as a chain (chain.cuh). Between ordinary launches the drain, the
+// launch and the set-up of the next kernel were 1-2 us of every 4: a training step at batch 2048 goes
+// from 158 to 134 us with the chain, a screen of 512 inputs from 41.8 to 33.6 us.
+using fb::launch_chain;
+using fb::pdl_chain;
 
 __device__ __forceinline__ uint16_t f2bf(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 
@@ -846,27 +839,6 @@ int cuda_status()
     if (e == cudaSuccess) return FB_OK;
     fb::set_last_error(cudaGetErrorString(e));
     return FB_ERR_CUDA;
-}
-
-// A launch of the chain (pdl_chain), as clusters of 1 x cy x cz blocks
-template <typename... P, typename... A>
-cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cy, unsigned cz, A... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = 1;
-    at[1].val.clusterDim.y = cy;
-    at[1].val.clusterDim.z = cz;
-    cfg.attrs = at;
-    cfg.numAttrs = cy * cz > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 template <int BN>
