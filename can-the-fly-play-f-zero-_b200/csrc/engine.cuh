@@ -1,5 +1,5 @@
 // Device-resident layout of one engine (a connectome shared by B instances) and the
-// two-launches-per-step kernels. Layout in HBM:
+// step engine's kernels. Layout in HBM:
 //
 //   connectome  rowptr[n+1] i64 (rows padded to 8 entries), col[nnz_pad] i32,
 //               cnt[nnz_pad] i16 (INT32 mode) or wfx[nnz_pad] i64 (Q32.32 mode)
@@ -10,8 +10,8 @@
 //   state       v[B][n], g[B][n] (f32 or f64), ref[B][n] i8
 //   inputs      ext_idx[n] i32, p_ext[B][n_ext] f32, bias_ext[B][n_ext] f32
 //   delay line  acc[S][B][n_pad] (i32 or i64): synaptic input of the next S ticks (slot = tick mod
-//               S, S = 2 x the persistent engine's epoch, at least 2), rows padded to 16 entries so
-//               that every row starts on a 64-byte boundary (TMA bulk copies);
+//               S, S = 2 x the persistent engine's epoch, at least 2), rows padded to 16 entries
+//               so that every row starts on a 16-byte boundary at any accumulator width;
 //               items[R][n_groups][cap_c] int2: spike work lists of the last R = n_delay + K steps (K: the
 //               persistent engine's epoch, 1 without it; a list is emptied K steps before it is filled
 //               again), one per instance group; item_count[R][n_groups];
@@ -407,16 +407,21 @@ __device__ __forceinline__ void push_lists(const DevNet& N, const DevState& S, i
 
 // ---------------------------------------------------------------------------------------------
 // Step engine: one launch per step. The first n_push blocks scatter the spikes that arrive at t+1, the
-// others advance every (instance, neuron) through step t, `per` blocks an instance. The two touch
+// others advance every (instance, neuron) through step t, `per` blocks an instance and `tiles` pairs a thread. The two touch
 // different accumulator slots (t+1 and t) and, with n_delay >= 2, different lists: the pushed one
 // (step t+1-n_delay) was filled by an earlier launch, the one that starts empty here held step t-n_delay,
 // pushed by the launch before. With n_delay = 1 the pushed spikes are this step's own, so the host
 // launches the two parts one after the other (n_push = 0, then pushing blocks alone).
 // `do_push` 0: the arrivals of t+1 were pushed ahead already (by the persistent engine); only the mask
 // slot is cleared.
+// Small networks are bound by a launch's chain of dependent loads (list length, item, edges;
+// accumulator, state, kick): 16 x 16,384 FP64 took 14.6 us a step as two ordinary launches and takes 7.0,
+// 4 x 1,000 11.7 and 4.0. Large ones are bound by the state's traffic in L2: 16 x 138,639 FP64 30.7
+// and 22.8, 64 x 138,639 FP32 123 and 94.
 // ---------------------------------------------------------------------------------------------
 struct StepGrid {
     int32_t n_push, per;       // pushing blocks; updating blocks per instance
+    int32_t tiles;             // 256 neurons each of an updating block
     int32_t do_push, lanes;
 };
 
@@ -434,7 +439,9 @@ __global__ void __launch_bounds__(256) k_step(const __grid_constant__ DevNet N, 
     const int32_t b = (int32_t)(u / (uint32_t)G.per);
     if (u == 0)                // the lists consumed by the push at t-1 start empty again
         for (int32_t k = threadIdx.x; k < S.n_groups; k += blockDim.x) *count_of(S, pos_mod(A.t - N.n_delay, N.R), k) = 0;
-    update_pair<Real, AccT, RASTER, PLASTIC, RECORD>(N, S, A, b, (int64_t)(u % (uint32_t)G.per) * blockDim.x + threadIdx.x);
+    const int64_t i0 = (int64_t)(u % (uint32_t)G.per) * G.tiles * 256 + threadIdx.x;
+#pragma unroll 1
+    for (int k = 0; k < G.tiles; k++) update_pair<Real, AccT, RASTER, PLASTIC, RECORD>(N, S, A, b, i0 + k * 256);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -54,6 +54,13 @@ def test_step_launches_match_the_oracle(n, B, delay, integral, real):
     gb.check()
 
 
+def test_several_tiles_per_block():
+    gb, eo = _pair(20_011, 61, 1.8, np.float32, True)          # 79 x 61 tiles: two for each block, the last one ragged
+    gb.set_schedule("step", lanes=8)
+    _same(gb, eo, gb.run_steps(40), eo.run_steps(40))
+    gb.check()
+
+
 @pytest.mark.parametrize("delay", [0.1, 0.2, 1.8])
 def test_pull_between_pushes(delay):
     gb, eo = _pair(777, 4, delay, np.float64, True)
