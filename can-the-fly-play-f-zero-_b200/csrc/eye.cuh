@@ -22,6 +22,7 @@
 //                  instance's restart flag.
 // One rounding per operation in the order NumPy evaluates it, no contraction.
 #pragma once
+#include "chain.cuh"
 #include "common.cuh"
 
 namespace fb {
@@ -303,6 +304,7 @@ __device__ __forceinline__ void cell_sums(const EyeArgs& a, const uint8_t* fr, b
 template <bool VEC4>
 __global__ void __launch_bounds__(256) k_eye_grid(const EyeArgs a)
 {
+    pdl_chain();
     const int64_t cells = (int64_t)a.gh * a.gw;
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (int64_t)a.B * cells) return;
@@ -376,6 +378,7 @@ __device__ __forceinline__ void running_sum(float* v, int32_t n, int32_t stride)
 
 __global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, const EyeSmem S, int32_t run)
 {
+    pdl_chain();
     extern __shared__ float sm[];
     __shared__ int32_t s_kind[4];                                  // neurons of each kind in the chunk
     const int32_t b = blockIdx.y, W1 = a.gw + 1, tid = threadIdx.x, lane = tid & 31;
