@@ -7,10 +7,10 @@ contrast U[0.2, 1], tonic DNp09 drive U[20, 100] Hz, run length U{0.5, 1, 2, 3} 
 plastic weights on the 7,300 inputs of 8 motor neurons. One bench step = one 166-step frame
 (16.64 ms at dt = 0.1 ms) for every instance, i.e. BatchBrain.run(16.64) after the frame's rates
 are written (flyzero/fleet.py:74-81). Inputs (per-frame rates) are resident in HBM before the
-timed region; the working set (state 80 MB + accumulators 71 MB + CSR 94 MB) exceeds the 126 MB L2.
+timed region; the working set (state 80 MB + accumulators 213 MB + CSR 94 MB) exceeds the 126 MB L2.
 
 Also reported in the same line: the roofline of the dominant kernel, the plain single-instance
-engine (B=1, two launches per step), the end-to-end path through the public API with host buffers,
+engine (B=1, one launch per step), the end-to-end path through the public API with host buffers,
 and the CPU oracle port timed on this host. ``--impl reference`` times the CPU port of the
 reference kernel (flyzero/brain.py:32-58) on all host cores, one instance per thread.
 """
@@ -486,7 +486,7 @@ def run_ours(args, world, rank, local):
                                   "first run; ended runs are reset and restarted at the next frame",
                    "runs_restarted_in_timed_loop": loop.reset_instances - reset_inst0,
                    "frames_with_restarts": loop.resets - resets0,
-                   "l2": "no flush: working set (state 80 MB + accumulators 71 MB + CSR 94 MB) exceeds the 126 MB L2",
+                   "l2": "no flush: working set (state 80 MB + accumulators 213 MB + CSR 94 MB) exceeds the 126 MB L2",
                    "spikes": spk, "mean_rate_hz": spk / max(1, active) / (DT / 1000.0) / n * 1.0},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
@@ -541,7 +541,7 @@ def persistent_b1(conn, drive, dev, frames: int = 6):
 
 
 def plain_b1(conn, drive, dev, frames: int = 6):
-    """The plain single-instance engine: B=1, two launches per step, no persistence, no graph."""
+    """The plain single-instance engine: B=1, one launch per step, no persistence, no graph."""
     import torch
 
     from flyzero_b200 import workloads as wl
@@ -563,7 +563,7 @@ def plain_b1(conn, drive, dev, frames: int = 6):
     b.record(st)
     torch.cuda.synchronize(dev)
     ms = a.elapsed_time(b)
-    return {"value": frames * fs * conn.n / (ms / 1000.0), "unit": UNIT, "engine": "step, B=1, 2 launches/step",
+    return {"value": frames * fs * conn.n / (ms / 1000.0), "unit": UNIT, "engine": "step, B=1, 1 launch/step",
             "ms_per_frame": ms / frames, "spikes_last_frame": int(c.sum())}
 
 
@@ -865,7 +865,7 @@ def run_fleet(args, world, rank, local):
                                f"neurons) -> {fs} LIF steps at dt 0.1 ms -> readout of 9 DN groups -> buttons",
                    "batch": B, "steps_per_frame": fs, "parallelism": f"replicas x{world}",
                    "frames_per_s": B * args.steps / (max_ms / 1000.0), "buttons_pressed": int(pressed),
-                   "l2": "no flush: the brain's working set (state 80 MB + accumulators 71 MB + CSR 94 MB) "
+                   "l2": "no flush: the brain's working set (state 80 MB + accumulators 213 MB + CSR 94 MB) "
                          "exceeds the 126 MB L2"},
         "gpu_launches": gb.launches - l0,
         "clocks": clk,

@@ -22,8 +22,9 @@
 //
 // The delay line is "deferred push": the fixed-weight rows of the spikes of step s are scattered
 // into acc only shortly before they arrive (the step engine at step s + n_delay - 1, the
-// persistent engine one epoch ahead), so only S accumulator slots (instead of n_delay) are live. Fixed weights never change during a run and integer addition is
-// order-free, so this equals the reference's push-at-spike-time ring (brain.py:54-56) exactly.
+// persistent engine one epoch ahead), so only S accumulator slots (instead of n_delay) are live.
+// Fixed weights never change during a run and integer addition is order-free, so this equals the
+// reference's push-at-spike-time ring (brain.py:54-56) exactly.
 // Plastic weights may change between runs, so their rows are pushed at spike time.
 #pragma once
 #include "chain.cuh"

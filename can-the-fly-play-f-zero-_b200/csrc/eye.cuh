@@ -2,6 +2,9 @@
 // instance at once, writing the eye neurons' Poisson probabilities straight into p_ext: the
 // frames are already on the device, so no rates cross the bus and no host loop runs per frame.
 //
+// The default is two launches: k_eye_grid (a thread per instance and grid cell: luminance, high-pass,
+// delay arms, colours) and k_eye_neurons (several blocks per instance, its grids in shared memory). Grids
+// too large for that take four grid-wide kernels, which state the steps one by one:
 //   k_eye_cells    one thread per (instance, grid cell):
 //                  lum = mean over the cell x cell block of mean(R, G, B) / 255 (vision.py:136-140),
 //                  each block row summed with NumPy's pairwise rule, the row sums added in order;
@@ -225,7 +228,8 @@ __global__ void k_eye_delay(const EyeArgs a)
 // ---- the same eye in two launches (the default) ----------------------------------------------------------
 // The grid of every instance by one thread per cell, then the neurons of an instance by several blocks.
 // One block per instance (its grid in shared memory) kept 64 instances on 64 of the 148 SMs and waited
-// through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16.5.
+// through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16.5,
+// 23.3 together as a dependent chain (26.6 as ordinary launches).
 
 // x / 3 and x / 255 rounded to nearest for the values a pixel can take (R + G + B and its third, a byte): one
 // Newton correction of the quotient by its exact remainder (Markstein 1990). Checked against the

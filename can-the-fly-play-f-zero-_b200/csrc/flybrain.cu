@@ -374,7 +374,6 @@ int largest_input(fb_brain* h, int64_t* out)
     return FB_OK;
 }
 
-
 // Build what pull propagation needs: the connectome by postsynaptic neuron and the spike-mask
 // ring (zeroed; masks are recorded from the current step on). The device must be idle.
 int enable_pull(fb_brain* h)
@@ -468,9 +467,9 @@ extern "C" int fb_create(const fb_params* P, const int64_t* indptr, const int32_
     TRY(dalloc(&h->abort_flag, 1, tb));
     int dev_sms2 = h->sm_count;
     h->plan = plan_persistent(h->n, h->n_pad, h->B, h->f64 != 0, h->n_ref, h->n_delay, dev_sms2, h->device);
-    // the persistent engine runs epochs of K steps between grid barriers: the spikes of an epoch, listed
-    // in the next one, arrive three epochs later at the earliest when 3K <= n_delay; 2K accumulator slots
-    // its accumulators are 16 bits wide if no neuron's input can leave them in any step (all its presynaptic
+    // the persistent engine runs epochs of K steps between grid barriers, on 2K accumulator slots: the spikes of
+    // an epoch, listed in the next one, arrive three epochs later at the earliest when 3K <= n_delay.
+    // Its accumulators are 16 bits wide if no neuron's input can leave them in any step (all its presynaptic
     // neurons firing at once): half the bytes to read, clear and keep in L2
     int64_t largest = 0;
     if (h->plan.group > 0 && h->acc_mode == 0) TRY(largest_input(h, &largest));

@@ -264,7 +264,8 @@ class BatchBrain:
 
     def set_schedule(self, engine: str | None = None, propagation: str | None = None, lanes: int = 0):
         """engine: 'auto' | 'step' | 'persistent'; propagation: 'push' | 'pull' (pull runs on the step
-        engine; its first n_delay steps after the switch still push); lanes: 8/16/32 per work item."""
+        engine; its first n_delay steps after the switch still push); lanes: 8/16/32 per work item of the step
+        engine."""
         e = {None: 0, "auto": 0, "step": 1, "persistent": 2}[engine]
         pr = {None: -1, "push": 0, "pull": 1}[propagation]
         _lib.check(self._L.fb_set_schedule(self._h, e, pr, int(lanes)))

@@ -37,7 +37,7 @@ extern "C" {
 
 /* schedule: engine kinds */
 #define FB_ENGINE_AUTO 0
-#define FB_ENGINE_STEP 1         /* two launches per simulated step (update, propagate) */
+#define FB_ENGINE_STEP 1         /* one launch per simulated step (two with a delay of one step, and to pull) */
 #define FB_ENGINE_PERSISTENT 2   /* one persistent launch per run; state kept on chip */
 /* schedule: propagation kinds */
 #define FB_PROP_PUSH 0           /* scatter each spiking row into the accumulator (atomics) */
@@ -60,7 +60,7 @@ typedef struct {
     int32_t f64;          /* 1 for FP64 state */
     int32_t engine;       /* current schedule (FB_ENGINE_*) */
     int32_t propagation;  /* FB_PROP_* */
-    int32_t lanes;        /* lanes per spike work item (8, 16 or 32) */
+    int32_t lanes;        /* the step engine's lanes per spike work item (8, 16 or 32) */
     int32_t group;        /* instances per persistent group (0: persistent engine unavailable) */
     int32_t ctas;         /* CTAs of the persistent launch */
     int64_t n_plastic;    /* plastic CSR entries */
@@ -231,7 +231,7 @@ int fb_motion_eye(fb_brain* brain, const uint8_t* frames, int32_t H, int32_t W, 
                   const int32_t* gy, const uint8_t* chan, const uint8_t* visible, const int32_t* slot, float* rates,
                   void* stream);
 
-/* Choose the schedule (FB_ENGINE_*, FB_PROP_*, lanes per work item 8/16/32; 0 keeps a field). */
+/* Choose the schedule (FB_ENGINE_*, FB_PROP_*, the step engine's lanes per work item 8/16/32; 0 keeps a field). */
 int fb_set_schedule(fb_brain* brain, int32_t engine, int32_t propagation, int32_t lanes);
 
 /* Phase trace of the persistent engine (diagnostics). `trace` [device] holds `capacity` int64;
