@@ -482,8 +482,7 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
 
 // The pair-by-pair advance of up to 8 quads through the kc steps of the epoch whose first is s0, four
 // lanes per quad (`quad`: this lane's, or -1): the quads that the tiles' advance passes over because
-// they have a plastic target or a bias, a kick or a spike in this epoch, or because their instance
-// stops in it. Every load of the epoch is issued before the first step; what was read is cleared.
+// they have a plastic target or a bias, or a kick or a spike in this epoch. Every load of the epoch is issued before the first step; what was read is cleared.
 template <typename AccT, bool PLASTIC, bool RECORD, int KB>
 __device__ __noinline__ void advance_pairs(const PersistParams& P, int32_t quad, int32_t s0, int32_t kc, int par, int slot0,
                                            int ring0)
@@ -551,8 +550,10 @@ __device__ __noinline__ void advance_pairs(const PersistParams& P, int32_t quad,
     if (hits) record_spikes<PLASTIC, RECORD>(P, par, k, s0, hits);
 }
 
-// The advance of this CTA's tiles through the kc steps of the epoch whose first is s0 (FULL: kc = KB), a
-// quad of consecutive pairs per lane. The arithmetic is lif_step's without kicks, plastic input,
+// The advance of this CTA's tiles through the kc steps of the epoch whose first is s0 (FULL: kc = KB, and no
+// instance stops in it or has stopped), a quad of consecutive pairs per lane. Quads of an instance that
+// stops take their own number of steps here: handed to advance_pairs, they made every epoch after
+// the stop slow (a frame of 16 whole brains in which one run ends: 2.0 ms against 0.8). The arithmetic is lif_step's without kicks, plastic input,
 // biases and spikes, in straight-line code: the refractory counters of the whole epoch are known at
 // its start, and a quad that takes a kick or reaches the threshold (one in thirty) is left as it was
 // and handed to advance_pairs, together with those that do not qualify from the start. Testing for
@@ -567,7 +568,6 @@ __device__ __forceinline__ void advance_tiles(const PersistParams& P, int32_t tu
     PersistCnt* C = smem_at<PersistCnt>(P.lay.misc);
     const int lane = threadIdx.x & 31;
     const int32_t np = (int32_t)P.N.n_pad, end = first_turn + (cnt + TILE - 1) / TILE;
-    const bool stops = C->stops[par] != 0;
     AccT* slot[KB];                                             // this CTA's accumulators at each step
 #pragma unroll
     for (int s = 0; s < KB; s++) {
@@ -580,16 +580,15 @@ __device__ __forceinline__ void advance_tiles(const PersistParams& P, int32_t tu
     struct Ahead {
         Acc4 x[KB];
         uint32_t rb;                                            // the four refractory counters
-        bool ok, late;                                          // advanced here; its instance stops in the epoch
+        int32_t on;                                             // steps of the epoch that its instance advances (!FULL)
+        bool ok;                                                // advanced here
     };
     auto fetch = [&](Ahead& a, int32_t k) {
         a.rb = k < cnt ? *smem_at<uint32_t>(P.lay.ref + k) : 0xc0u;
         a.ok = !(a.rb & 0xc0c0c0c0u);                           // neither a special quad nor padding
-        a.late = false;
-        if (stops && a.ok) {
-            const int32_t bl = (int32_t)((uint32_t)(first_pair(P) + k) / (uint32_t)np);
-            if (smem_at<int32_t>(P.lay.ticks + 1024)[par * 64 + bl] < kc) { a.ok = false; a.late = true; }
-        }
+        a.on = kc;
+        if (!FULL && a.ok)
+            a.on = smem_at<int32_t>(P.lay.ticks + 1024)[par * 64 + (int32_t)((uint32_t)(first_pair(P) + k) / (uint32_t)np)];
 #pragma unroll
         for (int s = 0; s < KB; s++) {
             a.x[s].zero();
@@ -616,7 +615,7 @@ __device__ __forceinline__ void advance_tiles(const PersistParams& P, int32_t tu
                 k_next = (turn - first_turn) * TILE + 4 * lane;
                 fetch(next, k_next);
             }
-            bool aside = a.late;                                // for advance_pairs
+            bool aside = false;                                 // for advance_pairs
             if (a.ok) {
                 const float4 v4 = *smem_at<float4>(P.lay.v + 4 * k), g4 = *smem_at<float4>(P.lay.g + 4 * k);
                 const uint32_t kick = *smem_at<uint32_t>(P.lay.kick + par * ((P.per + 3) / 4) * 4 + k);
@@ -627,7 +626,7 @@ __device__ __forceinline__ void advance_tiles(const PersistParams& P, int32_t tu
                 float top = L.v_rest;
 #pragma unroll
                 for (int s = 0; s < KB; s++) {
-                    if (!FULL && s >= kc) break;
+                    if (!FULL && s >= a.on) break;
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         g[j] = fma_rn(g[j], L.ds, acc_to_real<float>(a.x[s].at(j), L.w_syn));
@@ -640,7 +639,7 @@ __device__ __forceinline__ void advance_tiles(const PersistParams& P, int32_t tu
                 if (!aside) {
                     *smem_at<float4>(P.lay.v + 4 * k) = make_float4(v[0], v[1], v[2], v[3]);
                     *smem_at<float4>(P.lay.g + 4 * k) = make_float4(g[0], g[1], g[2], g[3]);
-                    if (a.rb) *smem_at<uint32_t>(P.lay.ref + k) = __vsubus4(a.rb, 0x01010101u * (uint32_t)kc);
+                    if (a.rb) *smem_at<uint32_t>(P.lay.ref + k) = __vsubus4(a.rb, 0x01010101u * (uint32_t)(FULL ? kc : a.on));
 #pragma unroll
                     for (int s = 0; s < KB; s++)
                         if ((FULL || s < kc) && a.x[s].any()) Acc4::clear(slot[s] + k);
@@ -814,7 +813,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
                                                      slot0, ring0);
         }
         uint16_t* ev = smem_at<uint16_t>(P.lay.events) + (tid >> 5) * EV_BUF;   // this warp's quads for advance_pairs
-        if (kc == KB) advance_tiles<AccT, PLASTIC, RECORD, KB, true>(P, turn, sp_turns, ev, cnt, kc, ep0, par, slot0, ring0);
+        if (kc == KB && !C->stops[par]) advance_tiles<AccT, PLASTIC, RECORD, KB, true>(P, turn, sp_turns, ev, cnt, kc, ep0, par, slot0, ring0);
         else advance_tiles<AccT, PLASTIC, RECORD, KB, false>(P, turn, sp_turns, ev, cnt, kc, ep0, par, slot0, ring0);
         if (tid == PT - 1 && A.trace) {                         // the epoch's span, divided between its steps
             const long long d = max((clock64() - c_begin) / kc, 2LL);

@@ -155,3 +155,23 @@ def test_input_sums_at_the_edge_of_sixteen_bits(torch, top):
             eo.reset_flies([0, 2])
         _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps))
     gb.check()
+
+
+@pytest.mark.parametrize("integral", [True, False], ids=["counts", "float"])
+@pytest.mark.parametrize("n,B,delay", [(127, 9, 1.8), (1003, 63, 1.8), (2001, 5, 0.5), (30_011, 6, 1.8)])
+def test_stops_at_every_step_of_an_epoch(torch, n, B, delay, integral):
+    """Instances that stop before, at and inside the epochs of a run, among others that do not: each takes its own
+    number of steps of an epoch, and a stopped one stays as it was."""
+    gb, eo = _pair(torch, n, B, delay, integral=integral, plastic=0.05, bias=0.03)
+    _same(gb, eo, gb.run_steps(25), eo.run_steps(25))
+    left = np.where(np.arange(B) % 5 == 4, -1, np.arange(B) % 29)
+    gb.set_run_length(left)
+    stop = np.where(left < 0, 2 ** 62, eo.t + left).astype(np.int64)
+    for steps in (16, 1, 20):
+        _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps, stop_tick=stop))
+    ended = np.flatnonzero(left >= 0)
+    gb.reset(ended)
+    eo.reset_flies(list(ended))
+    gb.set_run_length(np.full(B, -1))
+    _same(gb, eo, gb.run_steps(31), eo.run_steps(31))
+    gb.check()
