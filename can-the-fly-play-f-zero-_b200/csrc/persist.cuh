@@ -13,7 +13,7 @@
 //             steps. The pairs are taken in tiles of 128 from a shared counter;
 //   list      (LIST_WARPS) the spikes of epoch e - 1: counts, plastic rows, and the work items of
 //             the group's list of each step;
-//   push      (PUSH_WARPS) the work items that arrive in [T + K, T + 2K), into the other K of the 2K
+//   push      (PUSH_WARPS, or BUSY_PUSH_WARPS) the work items that arrive in [T + K, T + 2K), into the other K of the 2K
 //             accumulator slots (slot = tick mod 2K). The items were listed in epoch e - 1 at the
 //             latest: T + 2K - 1 - n_delay < T - K.
 // The listing and pushing warps take tiles too when they are done. One grid barrier ends an epoch;
@@ -46,7 +46,8 @@ constexpr int K_BITS = 18;              // bits of a local pair index (per < 2^1
 
 constexpr int PUSH_WARPS = 5;                              // warps that scatter arriving items ...
 constexpr int LIST_WARPS = 2;                              // ... and that list the previous epoch's spikes
-constexpr int PUSH_THREADS = 32 * PUSH_WARPS;
+constexpr int BUSY_PUSH_WARPS = 7;                         // scattering warps in an epoch that follows one with ...
+constexpr int BUSY_ITEMS = 200;                            // ... more arriving items than this for its CTA
 constexpr int LIST_THREADS = 32 * LIST_WARPS;
 
 struct PersistPlan {
@@ -176,6 +177,7 @@ struct PersistCnt {
     int32_t stops[2];                        // an instance stops in (or before) the epoch (epoch parity)
     int32_t tile[2];                         // next tile (epoch parity)
     int32_t n_spk[2];                        // spikes buffered (epoch parity)
+    int32_t busy[2];                         // the last epoch scattered more than BUSY_ITEMS items (epoch parity)
     int32_t stop;
     int32_t cursor[MAX_EPOCH], base[MAX_EPOCH];  // a listing batch's items per step, and where they start in the lists
 };
@@ -419,9 +421,14 @@ __device__ __noinline__ void draw_kicks(const PersistParams& P, int32_t s0, int 
 // contiguous run of the CTA's items: 32 items are loaded at once (one per lane; those of instances that
 // were reset or have stopped are dropped), then each is scattered by the whole warp, 8 entries per
 // lane. What bounds it is the reductions (~0.7 per SM clock): loads queue up behind them, so that more
-// rows in flight per warp, or more pushing warps, slow the advance by as much as they gain.
+// rows in flight per warp, or more pushing warps, slow the advance by as much as they gain (fleet of 64
+// whole brains, some 90 items per CTA and epoch: 3.24 ms with 5 warps, 3.54 with 7). Where a network
+// fires so much that pushing is the longest part, two more warps push after an epoch with more than
+// BUSY_ITEMS items (16 x 50,000 neurons, all driven at 100 Hz: 1.57 ms with 5 warps, 1.33 with 7, 1.36
+// with 9, 1.97 with 12; at 150 items they cost as much as they gain). Sums are whole numbers: who pushes
+// an item does not matter. `next`: the coming epoch's parity.
 template <typename AccT>
-__device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int64_t a1, int w, int n_w)
+__device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int64_t a1, int w, int n_w, int next)
 {
     constexpr unsigned FULL = 0xffffffffu;
     const DevNet& N = P.N;
@@ -446,6 +453,7 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
     const int64_t M = off[MAX_EPOCH], np = N.n_pad, slot_stride = (int64_t)N.B * np;
     AccT* acc0 = reinterpret_cast<AccT*>(S.acc) + (int64_t)P.b0 * np;
     const int32_t slot0 = (int32_t)pos_mod(a0, S.n_slots), list0 = (int32_t)pos_mod(a0 - N.n_delay, N.R);
+    if (w == 0 && lane == 0) smem_at<PersistCnt>(P.lay.misc)->busy[next] = M > BUSY_ITEMS;
     const int32_t j1 = (int32_t)(M * (w + 1) / n_w);
     for (int32_t j0 = (int32_t)(M * w / n_w); j0 < j1; j0 += 32) {
         int32_t start = 0, len = 0;
@@ -751,7 +759,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
     // An epoch is known by its first step: what else a warp needs between the routines is derived again
     // from the parameters, so that few registers stay live across the advance
     const int K = A.epoch;
-    const bool is_l = tid < LIST_THREADS, is_p = !is_l && tid < LIST_THREADS + PUSH_THREADS;
+    const bool is_l = tid < LIST_THREADS, may_p = !is_l && tid < LIST_THREADS + 32 * BUSY_PUSH_WARPS;
     const int n_slots = P.S.n_slots;
     int slot0 = (int)pos_mod(A.t0, n_slots);                    // accumulator slot of the epoch's first tick
     int ring0 = PLASTIC ? (int)pos_mod(A.t0, P.N.R_pl) : 0;     // ... and its slot of the plastic ring
@@ -763,7 +771,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
     {
         const int64_t a1 = min(A.t0 + K, A.t0 + A.steps + 1);
         if (A.pushed_until < a1) {
-            push_epoch<AccT>(P, A.pushed_until, a1, tid >> 5, PT / 32);
+            push_epoch<AccT>(P, A.pushed_until, a1, tid >> 5, PT / 32, 0);
             __syncthreads();
             bar_target += gridDim.x;
             if (tid == 0) {
@@ -792,12 +800,12 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
                 if (A.trace)
                     for (int32_t s = 0; s < kc; s++) stamp(A, ep0 + s, 8);
             }
-        } else if (is_p) {
+        } else if (may_p && tid < LIST_THREADS + 32 * (C->busy[par] ? BUSY_PUSH_WARPS : PUSH_WARPS)) {
             // the arrivals of the next epoch (and of the tick after the run) not pushed yet
             const int64_t end = A.t0 + A.steps + 1, T = A.t0 + ep0;
             const int64_t pa0 = max(A.pushed_until, min(T + K, end)), pa1 = min(T + 2 * K, end);
             if (tid == LIST_THREADS) stamp(A, ep0, 7);
-            if (pa0 < pa1) push_epoch<AccT>(P, pa0, pa1, (tid - LIST_THREADS) >> 5, PUSH_WARPS);
+            if (pa0 < pa1) push_epoch<AccT>(P, pa0, pa1, (tid - LIST_THREADS) >> 5, C->busy[par] ? BUSY_PUSH_WARPS : PUSH_WARPS, par ^ 1);
             if (tid == LIST_THREADS) stamp(A, ep0, 10);
         }
         // ---- advance: the special quads first (8 of them per turn), then the tiles ---------------------
