@@ -490,7 +490,8 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
 
 // The pair-by-pair advance of up to 8 quads through the kc steps of the epoch whose first is s0, four
 // lanes per quad (`quad`: this lane's, or -1): the quads that the tiles' advance passes over because
-// they have a plastic target or a bias, or a kick or a spike in this epoch. Every load of the epoch is issued before the first step; what was read is cleared.
+// they have a plastic target or a bias, or a kick or a spike in this epoch. Every load of the epoch is
+// issued before the first step; what was read is cleared.
 template <typename AccT, bool PLASTIC, bool RECORD, int KB>
 __device__ __noinline__ void advance_pairs(const PersistParams& P, int32_t quad, int32_t s0, int32_t kc, int par, int slot0,
                                            int ring0)
