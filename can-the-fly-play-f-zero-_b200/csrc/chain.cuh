@@ -16,6 +16,14 @@ __device__ __forceinline__ void pdl_chain()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The same for a kernel whose successor reads, before its own wait, what was in memory before this kernel
+// began: the successor starts when all that has completed.
+__device__ __forceinline__ void pdl_chain_behind()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // A launch of such a chain, as clusters of 1 x cy x cz blocks
 template <typename... P, typename... A>
 cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cy, unsigned cz, A... args)

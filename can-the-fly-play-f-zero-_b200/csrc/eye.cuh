@@ -229,7 +229,9 @@ __global__ void k_eye_delay(const EyeArgs a)
 // The grid of every instance by one thread per cell, then the neurons of an instance by several blocks.
 // One block per instance (its grid in shared memory) kept 64 instances on 64 of the 148 SMs and waited
 // through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16.5,
-// 23.3 together as a dependent chain (26.6 as ordinary launches).
+// 22.0 together as a dependent chain whose second kernel reads its tables beside the first (23.3 without
+// that, 26.6 as ordinary launches). Small eyes lose a little by the second launch: 30 of 1,000 cells and 3,287
+// neurons 12.0 us a call against 10.8.
 
 // x / 3 and x / 255 rounded to nearest for the values a pixel can take (R + G + B and its third, a byte): one
 // Newton correction of the quotient by its exact remainder (Markstein 1990). Checked against the
@@ -308,7 +310,7 @@ __device__ __forceinline__ void cell_sums(const EyeArgs& a, const uint8_t* fr, b
 template <bool VEC4>
 __global__ void __launch_bounds__(256) k_eye_grid(const EyeArgs a)
 {
-    pdl_chain();
+    pdl_chain_behind();
     const int64_t cells = (int64_t)a.gh * a.gw;
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (int64_t)a.B * cells) return;
@@ -382,7 +384,6 @@ __device__ __forceinline__ void running_sum(float* v, int32_t n, int32_t stride)
 
 __global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, const EyeSmem S, int32_t run)
 {
-    pdl_chain();
     extern __shared__ float sm[];
     __shared__ int32_t s_kind[4];                                  // neurons of each kind in the chunk
     const int32_t b = blockIdx.y, W1 = a.gw + 1, tid = threadIdx.x, lane = tid & 31;
@@ -408,7 +409,8 @@ __global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, co
             if (x >= 0 && x < a.gw && y >= 0 && y < a.gh && c < EYE_CHANNELS && slot[u] >= 0 && slot[u] < a.n_ext) cell[u] = y * a.gw + x;
         }
     };
-    fetch(blockIdx.x * run);
+    fetch(blockIdx.x * run);                                       // (the caller's tables: they are older than k_eye_grid)
+    pdl_chain();
     {
         const float* hp = a.sig + (int64_t)b * 2 * cells;
         const float* off = a.ii + (int64_t)b * (a.gh + 1) * W1;

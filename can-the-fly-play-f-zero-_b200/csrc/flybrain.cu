@@ -816,21 +816,14 @@ extern "C" int fb_motion_eye(fb_brain* h, const uint8_t* frames, int32_t H, int3
     if (ep->kernels != 2 && floats * 4 <= 227 * 1024 && h->B <= 65535) {
         const unsigned blocks = (unsigned)((cells + 255) / 256);
         const bool wide = ep->cell == 4 && W % 4 == 0 && ((uintptr_t)frames & 3) == 0;
-        // a chain where the device is the longer part; below that a call is bound by the host, and an ordinary
-        // launch is the cheaper one to enqueue (30 eyes of 3,287 neurons: 12.0 us a call as a chain)
-        const bool chain = (int64_t)h->B * n_cells > 200000;
-        if (chain) launch_chain(wide ? k_eye_grid<true> : k_eye_grid<false>, blocks, 256, 0, st, 1, 1, a);
-        else if (wide) k_eye_grid<true><<<blocks, 256, 0, st>>>(a);
-        else k_eye_grid<false><<<blocks, 256, 0, st>>>(a);
+        launch_chain(wide ? k_eye_grid<true> : k_eye_grid<false>, blocks, 256, 0, st, 1, 1, a);
         CU(cudaGetLastError());
         // blocks per instance: enough to fill the SMs once, at least EYE_THREADS neurons each
         const EyeSmem S((int32_t)grid, (int32_t)ii, sust, a.chromatic != 0);
         const int32_t per = std::max(1, std::min(h->sm_count / h->B, (n_cells + EYE_THREADS - 1) / EYE_THREADS));
         const int32_t run = std::max(1, (n_cells + per - 1) / per);
         if (S.total * 4 > 48 * 1024) CU(cudaFuncSetAttribute(k_eye_neurons, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total * 4));
-        const dim3 shape((unsigned)per, (unsigned)h->B);
-        if (chain) launch_chain(k_eye_neurons, shape, EYE_THREADS, (size_t)S.total * 4, st, 1, 1, a, S, run);
-        else k_eye_neurons<<<shape, EYE_THREADS, (size_t)S.total * 4, st>>>(a, S, run);
+        launch_chain(k_eye_neurons, dim3((unsigned)per, (unsigned)h->B), EYE_THREADS, (size_t)S.total * 4, st, 1, 1, a, S, run);
         CU(cudaGetLastError());
         h->launches += 2;
         return FB_OK;
