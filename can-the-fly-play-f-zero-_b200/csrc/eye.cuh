@@ -350,10 +350,11 @@ __global__ void __launch_bounds__(256) k_eye_grid(const EyeArgs a)
 // instruction issue (~200 a neuron, 60 of them the sort).
 constexpr int EYE_THREADS = 1024, EYE_UNROLL = 4, EYE_CHUNK = EYE_THREADS * EYE_UNROLL;
 
+constexpr int EYE_SMEM_MAX = 227 * 1024;                          // of a block, all of it dynamic: the kernel has no static arrays
 struct EyeSmem {                                                   // offsets in floats
-    int32_t hp, on, off, lum, ii, col, rate, order, total;
+    int64_t hp, on, off, lum, ii, col, rate, order, kind, total;
     EyeSmem() = default;
-    EyeSmem(int32_t cells, int32_t ii_cells, bool sust, bool chrom)
+    EyeSmem(int64_t cells, int64_t ii_cells, bool sust, bool chrom)
     {
         hp = 0;
         on = hp + cells;
@@ -363,7 +364,8 @@ struct EyeSmem {                                                   // offsets in
         col = ii + (sust ? ii_cells : 0);
         rate = col + (chrom ? 2 * cells : 0);
         order = rate + EYE_CHUNK;
-        total = order + EYE_CHUNK;
+        kind = order + EYE_CHUNK;
+        total = kind + 4;
     }
 };
 
@@ -385,12 +387,12 @@ __device__ __forceinline__ void running_sum(float* v, int32_t n, int32_t stride)
 __global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, const EyeSmem S, int32_t run)
 {
     extern __shared__ float sm[];
-    __shared__ int32_t s_kind[4];                                  // neurons of each kind in the chunk
     const int32_t b = blockIdx.y, W1 = a.gw + 1, tid = threadIdx.x, lane = tid & 31;
     const int32_t cells = a.gh * a.gw;
     float *s_hp = sm + S.hp, *s_on = sm + S.on, *s_off = sm + S.off, *s_lum = sm + S.lum, *s_ii = sm + S.ii;
     float *s_col = sm + S.col, *s_rate = sm + S.rate;
     uint32_t* s_order = reinterpret_cast<uint32_t*>(sm + S.order); // per sorted place: entry | channel << 12 | visible << 16
+    int32_t* s_kind = reinterpret_cast<int32_t*>(sm + S.kind);     // neurons of each kind in the chunk
     const bool sust = a.sustained != 0.0;
     const int32_t k1 = min(a.n_cells, (int32_t)(blockIdx.x + 1) * run);
     // a chunk's neurons, loaded ahead (the first one's beside the grids): cell (-1: out of range, or no neuron),

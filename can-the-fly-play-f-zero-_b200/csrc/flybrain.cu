@@ -811,20 +811,18 @@ extern "C" int fb_motion_eye(fb_brain* h, const uint8_t* frames, int32_t H, int3
     const bool sust = ep->sustained_gain != 0.0;
     const int64_t block = grid * (8 * sust + 4 * (5 + 2 * a.chromatic)) + ii * 4 * sust + (766 + 256) * 4;
     if (ep->kernels == 1 && block > 227 * 1024)
-        return fail(FB_ERR_ARG, "eye grid too large for the one-block-per-instance kernel");
-    const int64_t floats = grid * (3 + sust + 2 * a.chromatic) + ii * sust + 2 * EYE_CHUNK;
-    if (ep->kernels != 2 && floats * 4 <= 227 * 1024 && h->B <= 65535) {
-        const unsigned blocks = (unsigned)((cells + 255) / 256);
+        return fail(FB_ERR_ARG, "eye grid too large for one block's shared memory");
+    const EyeSmem S(grid, ii, sust, a.chromatic != 0);
+    if (ep->kernels != 2 && S.total * 4 <= EYE_SMEM_MAX && h->B <= 65535) {
         const bool wide = ep->cell == 4 && W % 4 == 0 && ((uintptr_t)frames & 3) == 0;
-        launch_chain(wide ? k_eye_grid<true> : k_eye_grid<false>, blocks, 256, 0, st, 1, 1, a);
-        CU(cudaGetLastError());
+        // before the first launch, so that a refusal would leave the filters as they were; to the most any eye
+        // needs, so that a concurrent call for a smaller one does not lower it
+        if (S.total * 4 > 48 * 1024) CU(cudaFuncSetAttribute(k_eye_neurons, cudaFuncAttributeMaxDynamicSharedMemorySize, EYE_SMEM_MAX));
+        CU(launch_chain(wide ? k_eye_grid<true> : k_eye_grid<false>, (unsigned)((cells + 255) / 256), 256, 0, st, 1, 1, a));
         // blocks per instance: enough to fill the SMs once, at least EYE_THREADS neurons each
-        const EyeSmem S((int32_t)grid, (int32_t)ii, sust, a.chromatic != 0);
         const int32_t per = std::max(1, std::min(h->sm_count / h->B, (n_cells + EYE_THREADS - 1) / EYE_THREADS));
         const int32_t run = std::max(1, (n_cells + per - 1) / per);
-        if (S.total * 4 > 48 * 1024) CU(cudaFuncSetAttribute(k_eye_neurons, cudaFuncAttributeMaxDynamicSharedMemorySize, S.total * 4));
-        launch_chain(k_eye_neurons, dim3((unsigned)per, (unsigned)h->B), EYE_THREADS, (size_t)S.total * 4, st, 1, 1, a, S, run);
-        CU(cudaGetLastError());
+        CU(launch_chain(k_eye_neurons, dim3((unsigned)per, (unsigned)h->B), EYE_THREADS, (size_t)S.total * 4, st, 1, 1, a, S, run));
         h->launches += 2;
         return FB_OK;
     }
