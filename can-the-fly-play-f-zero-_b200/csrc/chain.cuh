@@ -10,6 +10,11 @@ namespace fb {
 // and a block waits only for blocks that are already resident (with their TMEM): a successor starts
 // when all of its predecessor's blocks have come this far. Behind an ordinary launch or copy, and
 // before one, the order is the stream's as ever.
+//
+// What any earlier work of the stream may have written is read with plain loads: a kernel of the chain is
+// resident while its predecessors still write, so such data is not read-only for its lifetime, as __ldg
+// demands (the compiler may move an __ldg above the wait, and the read-only path may hold old contents).
+// __ldg is for what is written before the chain begins, as the connectome.
 __device__ __forceinline__ void pdl_chain()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -259,7 +259,7 @@ __device__ __forceinline__ void cell_sums(const EyeArgs& a, const uint8_t* fr, b
         for (int32_t yy = 0; yy < 4; yy++) {
             const uint32_t* p = reinterpret_cast<const uint32_t*>(fr + ((int64_t)(4 * y + yy) * a.W + c0) * 3);
 #pragma unroll
-            for (int j = 0; j < 3; j++) w[yy][j] = __ldg(p + j);
+            for (int j = 0; j < 3; j++) w[yy][j] = p[j];
         }
 #pragma unroll
         for (int32_t yy = 0; yy < 4; yy++) {

@@ -127,7 +127,7 @@ __device__ __forceinline__ void epilogue16(const Epi& e, int M, int N, int i, in
         }
     } else {
 #pragma unroll
-        for (int u = 0; u < 16; u++) z[u] = e.mode == FS_EPI_F32 ? v[u] : v[u] + __ldg(e.bias + j + u);
+        for (int u = 0; u < 16; u++) z[u] = e.mode == FS_EPI_F32 ? v[u] : v[u] + e.bias[j + u];
 #pragma unroll
         for (int u = 0; u < 16; u += 4) *reinterpret_cast<float4*>(e.out_f32 + o + u) = make_float4(z[u], z[u + 1], z[u + 2], z[u + 3]);
     }
