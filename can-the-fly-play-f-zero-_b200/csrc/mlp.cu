@@ -793,7 +793,7 @@ __global__ void k_to_bf16_t(const float* x, uint16_t* out, uint16_t* out_t, int 
 __global__ void __launch_bounds__(256) k_to_bf16_t4(const float* x, uint16_t* out, uint16_t* out_t, int rows, int cols, int ldt)
 {
     pdl_chain();
-    __shared__ uint16_t tile[64][64 + 4];              // [column][row]
+    __shared__ __align__(8) uint16_t tile[64][64 + 4]; // [column][row], read four rows (8 bytes) at a time
     const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64, lane = threadIdx.x & 15, w = threadIdx.x >> 4;
     float4 q[4];
 #pragma unroll
