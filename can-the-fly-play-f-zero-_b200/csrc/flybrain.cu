@@ -197,7 +197,8 @@ struct fb_brain {
     void* acc16 = nullptr;        // the same in 16 bits for the persistent engine, where every input sum fits
     bool live16 = false;          // the input in flight is in acc16 (acc is zero), else in acc (acc16 is zero)
     int32_t n_slots = 2;
-    int32_t epoch = 1;            // persistent engine: steps per grid barrier
+    EpochPlan epochs;             // persistent engine: steps between grid barriers
+    int32_t last_epoch = 1;       // ... of the last run (before the first: with late listing)
     int64_t pushed_until = 1;     // the arrivals of every tick < pushed_until are in acc
     int64_t* pring = nullptr;
     int2* items = nullptr;
@@ -467,16 +468,16 @@ extern "C" int fb_create(const fb_params* P, const int64_t* indptr, const int32_
     TRY(dalloc(&h->abort_flag, 1, tb));
     int dev_sms2 = h->sm_count;
     h->plan = plan_persistent(h->n, h->n_pad, h->B, h->f64 != 0, h->n_ref, h->n_delay, dev_sms2, h->device);
-    // the persistent engine runs epochs of K steps between grid barriers, on 2K accumulator slots: the spikes of
-    // an epoch, listed in the next one, arrive three epochs later at the earliest when 3K <= n_delay.
+    // the persistent engine runs epochs of K steps between grid barriers, on 2K accumulator slots (plan_epochs).
     // Its accumulators are 16 bits wide if no neuron's input can leave them in any step (all its presynaptic
     // neurons firing at once): half the bytes to read, clear and keep in L2
     int64_t largest = 0;
     if (h->plan.group > 0 && h->acc_mode == 0) TRY(largest_input(h, &largest));
     const bool narrow = h->plan.group > 0 && h->acc_mode == 0 && largest <= INT16_MAX;
-    h->epoch = h->plan.group > 0 ? persistent_epoch(h->plan, h->n_pad, h->n_delay, narrow ? 2 : (int)ab) : 1;
-    h->n_slots = 2 * h->epoch;
-    h->R_pl = h->R = h->n_delay + h->epoch;
+    if (h->plan.group > 0) h->epochs = plan_epochs(h->n_delay, narrow ? 2 : (int)ab);
+    h->last_epoch = h->epochs.late;
+    h->n_slots = 2 * h->epochs.steps;
+    h->R_pl = h->R = h->n_delay + h->epochs.steps;
     TRY(dalloc((char**)&h->acc, nbp * ab * h->n_slots, tb));
     CU(cudaMemset(h->acc, 0, nbp * ab * h->n_slots));
     if (narrow) {
@@ -543,7 +544,7 @@ extern "C" int fb_get_info(const fb_brain* h, fb_info* o)
     o->acc_mode = h->acc_mode; o->f64 = h->f64; o->engine = h->engine; o->propagation = h->prop;
     o->lanes = h->lanes; o->group = h->plan.group; o->ctas = h->plan.ctas; o->n_plastic = h->n_pl;
     o->n_ext = h->n_ext; o->t = h->t; o->step_no = h->step_no; o->launches = h->launches;
-    o->item_capacity = h->cap_c; o->bytes_device = (int64_t)h->bytes; o->epoch = h->epoch;
+    o->item_capacity = h->cap_c; o->bytes_device = (int64_t)h->bytes; o->epoch = h->last_epoch;
     o->decay_syn = h->consts64[0]; o->decay_m = h->consts64[1]; o->kick = h->consts64[2];
     return FB_OK;
 }
@@ -996,7 +997,8 @@ extern "C" int fb_run(fb_brain* h, int32_t steps, int32_t* counts_out, const uin
         P.bar = h->bar; P.abort_flag = h->abort_flag; P.ext_tab = h->ext_tab; P.ext_off = h->ext_off;
         P.trace = ((int64_t)steps * h->plan.ctas * TRACE_SLOTS <= h->trace_cap) ? h->trace : nullptr;
         P.pushed_until = h->pushed_until;
-        P.epoch = h->epoch;
+        P.epoch = h->last_epoch = h->epochs.steps;
+        P.list_late = 3 * P.epoch <= h->n_delay;
         P.barrier_cycles = h->barrier_cycles;
         CU(cudaMemsetAsync(h->abort_flag, 0, sizeof(int32_t), st));
         int rc = launch_persistent(h->plan, h->net(), h->state(), P, h->live16 ? 2 : h->acc_mode == 0 ? 4 : 8, h->n_pl > 0, kicks != nullptr, record,

@@ -5,17 +5,19 @@
 // GPU (148 x ~227 KB). Each CTA owns a contiguous slice of the group's (instance, neuron) pairs and
 // keeps their state in shared memory for the whole run.
 //
-// Epochs: the spikes of a step arrive n_delay steps later, so with 3K <= n_delay everything that
-// arrives during an epoch of K steps (at most MAX_EPOCH) is known one epoch ahead, with an epoch to
-// spare for listing. In epoch e, which covers the ticks [T, T + K), the warps of a CTA
+// Epochs: the spikes of a step arrive n_delay steps later, so with 2K <= n_delay everything that
+// arrives during an epoch of K steps (at most MAX_EPOCH) is known one epoch ahead, and with 3K <=
+// n_delay there is an epoch to spare for listing. In epoch e, which covers the ticks [T, T + K), the
+// warps of a CTA
 //   advance   every pair through all K steps at once: its K accumulator values are read from L2
 //             (and cleared), its state is loaded and stored once, and no barrier separates the
 //             steps. The pairs are taken in tiles of 128 from a shared counter;
 //   list      (LIST_WARPS) the spikes of epoch e - 1: counts, plastic rows, and the work items of
-//             the group's list of each step;
+//             the group's list of each step. With 3K > n_delay the whole CTA lists the epoch's own
+//             spikes after the advance instead: no list is late, and the epoch is 2-3 us longer;
 //   push      (PUSH_WARPS, or BUSY_PUSH_WARPS) the work items that arrive in [T + K, T + 2K), into the other K of the 2K
 //             accumulator slots (slot = tick mod 2K). The items were listed in epoch e - 1 at the
-//             latest: T + 2K - 1 - n_delay < T - K.
+//             latest: T + 2K - 1 - n_delay < T - K (< T where epochs list their own spikes).
 // The listing and pushing warps take tiles too when they are done. One grid barrier ends an epoch;
 // between arriving at it and waiting for it a CTA draws the next epoch's Poisson kicks.
 //
@@ -74,7 +76,8 @@ struct PersistArgs {
     const int32_t* ext_off;   // (ctas + 1) offsets into ext_tab
     long long* trace;         // nullptr, or (steps, ctas, TRACE_SLOTS) clock64 stamps of each step's phases
     int64_t pushed_until;     // the arrivals of every tick < pushed_until are in the accumulators
-    int32_t epoch;            // K: steps between grid barriers (2K accumulator slots, 3K <= n_delay)
+    int32_t epoch;            // K: steps between grid barriers (at most n_slots / 2, 2K <= n_delay or K = 1)
+    int32_t list_late;        // an epoch's spikes are listed in the next one (3K <= n_delay), else at its own end
     long long barrier_cycles; // the grid barrier's wait budget (SM clock cycles) before it times out
 };
 
@@ -749,11 +752,10 @@ __device__ __noinline__ void store_state(const PersistParams& P, int32_t cnt)
 template <typename AccT, bool RASTER, bool PLASTIC, bool RECORD, int KB>
 __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ PersistParams P)
 {
-    using Acc4 = typename Acc4Of<AccT>::T;
     const PersistArgs& A = P.A;
     PersistCnt* C = smem_at<PersistCnt>(P.lay.misc);
     const int tid = threadIdx.x, lane = tid & 31;
-    const int32_t n = (int32_t)P.N.n, np = (int32_t)P.N.n_pad;
+    const int32_t np = (int32_t)P.N.n_pad;
     const int32_t cnt = (int32_t)max((int64_t)0, min((int64_t)P.per, (int64_t)P.G * np - first_pair(P)));
     load_state<RASTER, PLASTIC, KB>(P, cnt);
 
@@ -791,7 +793,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
         if (tid == PT - 1 && A.trace) c_begin = clock64();
         if (is_l) {
             const int32_t kc = min(K, A.steps - ep0);
-            if (ep0 > 0) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, K, false);
+            if (A.list_late && ep0 > 0) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, K, false);
             // the lists whose items arrive in this epoch were pushed before it: they are empty when they are
             // filled again, K steps after the ticks of this epoch
             if (blockIdx.x == 0 && tid < kc) *count_of(P.S, pos_mod(A.t0 + ep0 + tid - P.N.n_delay, P.N.R), P.q) = 0;
@@ -837,6 +839,10 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
         if (slot0 >= n_slots) slot0 -= n_slots;
         ring0 += kc;
         if (ring0 >= P.N.R_pl) ring0 -= P.N.R_pl;
+        if (!A.list_late) {
+            __syncthreads();                                    // every spike of the epoch is buffered
+            list_epoch<PLASTIC, RECORD>(P, par, ep0, kc, true);
+        }
         if (ep0 + K < A.steps) {                                // another epoch follows
             __syncthreads();                                    // this epoch's work of the CTA is done
             long long c0 = 0;
@@ -858,7 +864,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
     }
     // the last epoch's spikes are listed before the launch ends (the next launch scatters them)
     __syncthreads();
-    if (!stop) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, A.steps - (ep0 - K), true);
+    if (!stop && A.list_late) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, A.steps - (ep0 - K), true);
     store_state(P, cnt);
 }
 
@@ -897,14 +903,23 @@ inline PersistPlan plan_persistent(int64_t n, int64_t n_pad, int32_t B, bool f64
     return P;
 }
 
-// Steps per epoch: 3K <= n_delay. Longer epochs mean fewer barriers, but the 2K accumulator slots of the
-// group are to stay in L2: in 16 bits K = 6 takes 53 MB for 16 whole brains (4.53 us per step, 4.80 with
-// K = 4); in 32 bits it takes 106 MB and was slower (7.9 us per step, 5.5 with K = 4).
-inline int persistent_epoch(const PersistPlan& P, int64_t n_pad, int n_delay, int acc_bytes)
+// Steps per epoch. Longer epochs mean fewer barriers, but the 2K accumulator slots of the group are to stay
+// in L2: in 16 bits K = 6 takes 53 MB for 16 whole brains (4.53 us per step, 4.80 with K = 4; 18 brains
+// 2.95 and 3.46); in 32 bits it takes 106 MB and was slower (7.9 us per step, 5.5 with K = 4).
+// Listing an epoch's spikes in the next one takes 3K <= n_delay, at its own end 2K <= n_delay and 2-3 us.
+// The longer epoch is worth it from a third more steps on: ms per 166 steps of 64 whole brains with
+// K = 1 late / 2 own 5.71 / 3.93, 2 / 3 3.39 / 2.98, 3 / 4 2.55 / 2.47, 4 / 6 2.16 / 2.05, but 5 / 6 1.98 / 2.05.
+struct EpochPlan {
+    int32_t late = 1;         // the longest that can be listed late
+    int32_t steps = 1;        // K of a run
+};
+inline EpochPlan plan_epochs(int n_delay, int acc_bytes)
 {
-    const int64_t slot = (int64_t)P.group * n_pad * acc_bytes;
-    const int most = acc_bytes == 2 && slot * 2 * MAX_EPOCH <= (int64_t)56 << 20 ? MAX_EPOCH : 4;
-    return std::max(1, std::min(most, n_delay / 3));
+    const int most = acc_bytes == 2 ? MAX_EPOCH : 4, own = std::min(most, n_delay / 2);
+    EpochPlan E;
+    E.late = std::max(1, std::min(most, n_delay / 3));
+    E.steps = 3 * own >= 4 * E.late ? own : E.late;
+    return E;
 }
 
 template <typename AccT, bool RASTER, bool PLASTIC, bool RECORD, int KB>
@@ -957,10 +972,14 @@ cudaError_t launch_persist_acc(const PersistPlan& P, const DevNet& N, const DevS
 inline cudaError_t launch_persistent(const PersistPlan& P, const DevNet& N, const DevState& S, const PersistArgs& A,
                                      int acc_bytes, bool plastic, bool raster, bool record, cudaStream_t st)
 {
-    if (acc_bytes == 8) return launch_persist_acc<int64_t, 4>(P, N, S, A, plastic, raster, record, st);
-    if (acc_bytes == 4) return launch_persist_acc<int32_t, 4>(P, N, S, A, plastic, raster, record, st);
-    if (A.epoch <= 4) return launch_persist_acc<int16_t, 4>(P, N, S, A, plastic, raster, record, st);
-    return launch_persist_acc<int16_t, MAX_EPOCH>(P, N, S, A, plastic, raster, record, st);
+    // KB = K: an advance with room for more steps than an epoch has takes the form for instances that stop, and
+    // reads and tests slots it does not use (64 whole brains, 166 steps at K = 2: 4.06 ms with KB = 4, 3.33 with 2)
+#define LK_(T_, K_) case K_: return launch_persist_acc<T_, K_>(P, N, S, A, plastic, raster, record, st)
+    if (acc_bytes == 8) switch (A.epoch) { LK_(int64_t, 1); LK_(int64_t, 2); LK_(int64_t, 3); LK_(int64_t, 4); }
+    if (acc_bytes == 4) switch (A.epoch) { LK_(int32_t, 1); LK_(int32_t, 2); LK_(int32_t, 3); LK_(int32_t, 4); }
+    if (acc_bytes == 2) switch (A.epoch) { LK_(int16_t, 1); LK_(int16_t, 2); LK_(int16_t, 3); LK_(int16_t, 4); LK_(int16_t, 5); LK_(int16_t, 6); }
+#undef LK_
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace fb

@@ -246,7 +246,7 @@ class BatchBrain:
             torch.cuda.synchronize(self.device)
         finally:
             _lib.check(self._L.fb_set_trace(self._h, None, 0))
-        return tr.cpu().numpy().reshape(steps, ctas, TRACE_SLOTS), int(info.epoch)
+        return tr.cpu().numpy().reshape(steps, ctas, TRACE_SLOTS), int(self.info().epoch)
 
     def make_plastic(self, pos):
         """Add CSR positions to the plastic set (keeps state and input in flight)."""

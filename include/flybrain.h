@@ -73,7 +73,8 @@ typedef struct {
     double decay_syn;     /* exp(-dt / tau_syn), computed in FP64 on the device */
     double decay_m;       /* dt / tau_m */
     double kick;          /* f_poisson * w_syn, mV */
-    int32_t epoch;        /* persistent engine: steps between grid barriers (accumulator slots = 2x) */
+    int32_t epoch;        /* persistent engine: steps between grid barriers in its last run (before the first:
+                           * the most that n_delay allows when a step's spikes are listed an epoch late) */
 } fb_info;
 
 /* Device views of the mutable state a caller may read and write between runs. */

@@ -41,7 +41,7 @@ def test_queued_steps_equal_synchronised_steps(torch, M):
     rng = np.random.default_rng(M)
     data = [(torch.as_tensor(rng.standard_normal((M, 1280)).astype(np.float32), device="cuda"),
              torch.as_tensor(rng.poisson(2.0, (M, 10)).astype(np.float32), device="cuda")) for _ in range(6)]
-    nets = [MLP(seed=1, lr=0.05), MLP(seed=1, lr=0.05)]            # (a rate that moves the biases in every step)
+    nets = [MLP(seed=1), MLP(seed=1)]
     nets[1].L = Synchronised(nets[1].L, torch)
     outs = []
     for net in nets:
