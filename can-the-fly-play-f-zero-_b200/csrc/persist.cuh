@@ -49,7 +49,8 @@ constexpr int K_BITS = 18;              // bits of a local pair index (per < 2^1
 constexpr int PUSH_WARPS = 5;                              // warps that scatter arriving items ...
 constexpr int LIST_WARPS = 2;                              // ... and that list the previous epoch's spikes
 constexpr int BUSY_PUSH_WARPS = 7;                         // scattering warps in an epoch that follows one with ...
-constexpr int BUSY_ITEMS = 200;                            // ... more arriving items than this for its CTA
+constexpr int BUSY_ENTRIES = 12000;                        // ... more arriving entries than this per step for its CTA
+constexpr int PUSH_LANES = 16;                             // lanes that scatter an item
 constexpr int LIST_THREADS = 32 * LIST_WARPS;
 
 struct PersistPlan {
@@ -180,7 +181,7 @@ struct PersistCnt {
     int32_t stops[2];                        // an instance stops in (or before) the epoch (epoch parity)
     int32_t tile[2];                         // next tile (epoch parity)
     int32_t n_spk[2];                        // spikes buffered (epoch parity)
-    int32_t busy[2];                         // the last epoch scattered more than BUSY_ITEMS items (epoch parity)
+    int32_t entries[2];                      // entries scattered in the last epoch (epoch parity)
     int32_t stop;
     int32_t cursor[MAX_EPOCH], base[MAX_EPOCH];  // a listing batch's items per step, and where they start in the lists
 };
@@ -422,13 +423,17 @@ __device__ __noinline__ void draw_kicks(const PersistParams& P, int32_t s0, int 
 // Push warps: this CTA's shares of the lists arriving at ticks [a0, a1) (at most MAX_EPOCH lists, the
 // spikes of n_delay ticks before) scattered into their accumulator slots. Warp w of n_w takes a
 // contiguous run of the CTA's items: 32 items are loaded at once (one per lane; those of instances that
-// were reset or have stopped are dropped), then each is scattered by the whole warp, 8 entries per
-// lane. What bounds it is the reductions (~0.7 per SM clock): loads queue up behind them, so that more
-// rows in flight per warp, or more pushing warps, slow the advance by as much as they gain (fleet of 64
-// whole brains, some 90 items per CTA and epoch: 3.24 ms with 5 warps, 3.54 with 7). Where a network
-// fires so much that pushing is the longest part, two more warps push after an epoch with more than
-// BUSY_ITEMS items (16 x 50,000 neurons, all driven at 100 Hz: 1.57 ms with 5 warps, 1.33 with 7, 1.36
-// with 9, 1.97 with 12; at 150 items they cost as much as they gain). Sums are whole numbers: who pushes
+// were reset or have stopped are dropped), then two at a time are scattered, each by half of the warp, 8
+// entries per lane: a row of 60 entries leaves 24 lanes of a warp idle, and a chain of loads and
+// reductions a row is what a warp waits for. ms per 166 steps of 16 x 50,000 neurons with 60 entries, all
+// driven at 100 Hz, by lanes an item and pushing warps: 32 lanes 1.58 (5 warps), 1.33 (7), 1.37 (9);
+// 16 lanes 1.14, 1.20, 1.41; 8 lanes 1.16, 1.27, 1.47. Rows of 110 entries do not mind (64 whole
+// brains 1.82 with 32 and 16 lanes, 1.85 with 8). More warps than 5 slow the advance by as much as they
+// gain, for their loads and its loads queue up behind the reductions (~0.7 per SM clock), until
+// pushing is by far the longest part. So two more warps push after an epoch with more than BUSY_ENTRIES a
+// step and CTA. ms with 5 and 7 warps, by entries: 35 thousand (16 whole brains, 30 % driven at 100 Hz) 9.9 and
+// 7.8; 15 thousand (16 x 20,000, 300 entries a row, all at 60 Hz) 2.35 and 2.18; 10 thousand (16 x 50,000, all
+// at 400 Hz) 2.29 and 2.29; 5 thousand (half of them) 1.38 and 1.60. Sums are whole numbers: who pushes
 // an item does not matter. `next`: the coming epoch's parity.
 template <typename AccT>
 __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int64_t a1, int w, int n_w, int next)
@@ -456,8 +461,8 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
     const int64_t M = off[MAX_EPOCH], np = N.n_pad, slot_stride = (int64_t)N.B * np;
     AccT* acc0 = reinterpret_cast<AccT*>(S.acc) + (int64_t)P.b0 * np;
     const int32_t slot0 = (int32_t)pos_mod(a0, S.n_slots), list0 = (int32_t)pos_mod(a0 - N.n_delay, N.R);
-    if (w == 0 && lane == 0) smem_at<PersistCnt>(P.lay.misc)->busy[next] = M > BUSY_ITEMS;
     const int32_t j1 = (int32_t)(M * (w + 1) / n_w);
+    int32_t mine = 0;
     for (int32_t j0 = (int32_t)(M * w / n_w); j0 < j1; j0 += 32) {
         int32_t start = 0, len = 0;
         int64_t to = 0;                                         // offset of the item's row of accumulators
@@ -475,20 +480,24 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
             if (a0 + k - N.n_delay >= s_reset[bl] && a0 + k < s_stop[bl]) len = item.y & ((1 << CHUNK_BITS) - 1);
             const int32_t sl = slot0 + k < S.n_slots ? slot0 + k : slot0 + k - S.n_slots;
             to = sl * slot_stride + (int64_t)bl * np;
+            mine += len;
         }
         const int n = min(32, j1 - j0);
-        for (int u = 0; u < n; u++) {
+        for (int u0 = 0; u0 < n; u0 += 32 / PUSH_LANES) {
+            const int u = u0 + lane / PUSH_LANES;               // (u = n <= 31 where n is odd: an item of length 0)
             const int32_t r = __shfl_sync(FULL, start, u), l = __shfl_sync(FULL, len, u);
             AccT* acc = acc0 + __shfl_sync(FULL, to, u);
-            if (8 * lane < l) {
+            for (int32_t q = 8 * (lane % PUSH_LANES); q < l; q += 8 * PUSH_LANES) {
                 Edges8<typename SumOf<AccT>::T> e;
-                e.load(N, (int64_t)(uint32_t)r + 8 * lane);
+                e.load(N, (int64_t)(uint32_t)r + q);
 #pragma unroll
                 for (int c = 0; c < 8; c++)
                     if (e.w[c] != 0) red_acc(acc + e.c[c], e.w[c]);
             }
         }
     }
+    mine = __reduce_add_sync(FULL, mine);
+    if (lane == 0 && mine) atomicAdd(&smem_at<PersistCnt>(P.lay.misc)->entries[next], mine);
 }
 
 // The pair-by-pair advance of up to 8 quads through the kc steps of the epoch whose first is s0, four
@@ -762,7 +771,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
     // An epoch is known by its first step: what else a warp needs between the routines is derived again
     // from the parameters, so that few registers stay live across the advance
     const int K = A.epoch;
-    const bool is_l = tid < LIST_THREADS, may_p = !is_l && tid < LIST_THREADS + 32 * BUSY_PUSH_WARPS;
+    const bool is_l = tid < LIST_THREADS;
     const int n_slots = P.S.n_slots;
     int slot0 = (int)pos_mod(A.t0, n_slots);                    // accumulator slot of the epoch's first tick
     int ring0 = PLASTIC ? (int)pos_mod(A.t0, P.N.R_pl) : 0;     // ... and its slot of the plastic ring
@@ -803,12 +812,12 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
                 if (A.trace)
                     for (int32_t s = 0; s < kc; s++) stamp(A, ep0 + s, 8);
             }
-        } else if (may_p && tid < LIST_THREADS + 32 * (C->busy[par] ? BUSY_PUSH_WARPS : PUSH_WARPS)) {
+        } else if (const int n_w = C->entries[par] > BUSY_ENTRIES * K ? BUSY_PUSH_WARPS : PUSH_WARPS; tid < LIST_THREADS + 32 * n_w) {
             // the arrivals of the next epoch (and of the tick after the run) not pushed yet
             const int64_t end = A.t0 + A.steps + 1, T = A.t0 + ep0;
             const int64_t pa0 = max(A.pushed_until, min(T + K, end)), pa1 = min(T + 2 * K, end);
             if (tid == LIST_THREADS) stamp(A, ep0, 7);
-            if (pa0 < pa1) push_epoch<AccT>(P, pa0, pa1, (tid - LIST_THREADS) >> 5, C->busy[par] ? BUSY_PUSH_WARPS : PUSH_WARPS, par ^ 1);
+            if (pa0 < pa1) push_epoch<AccT>(P, pa0, pa1, (tid - LIST_THREADS) >> 5, n_w, par ^ 1);
             if (tid == LIST_THREADS) stamp(A, ep0, 10);
         }
         // ---- advance: the special quads first (8 of them per turn), then the tiles ---------------------
@@ -848,6 +857,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
             long long c0 = 0;
             if (tid == 0) {
                 c0 = clock64();
+                C->entries[par] = 0;                            // (the coming epoch adds to it)
                 grid_arrive(A);
                 stamp(A, ep0 + K - 1, 5);
             }
