@@ -333,8 +333,9 @@ int install_plastic(fb_brain* h, const std::vector<int64_t>& pos)
 // map changes; the same table serves every group (pairs are numbered within a group).
 int build_ext_table(fb_brain* h)
 {
-    const PersistPlan& P = h->plan;
+    PersistPlan& P = h->plan;
     if (P.group == 0) return FB_OK;
+    int32_t most = 0;
     std::vector<int32_t> off(P.ctas + 1, 0);
     std::vector<int2> tab;
     const int64_t np = h->n_pad, total = (int64_t)P.group * np;
@@ -347,6 +348,8 @@ int build_ext_table(fb_brain* h)
         }
     }
     off[P.ctas] = (int32_t)tab.size();
+    for (int32_t c = 0; c < P.ctas; c++) most = std::max(most, off[c + 1] - off[c]);
+    plan_inputs(P, most);
     if (h->ext_tab) h->graveyard.push_back(h->ext_tab);
     if (h->ext_off) h->graveyard.push_back(h->ext_off);
     h->ext_tab = nullptr;

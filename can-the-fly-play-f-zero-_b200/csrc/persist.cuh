@@ -41,7 +41,7 @@ constexpr int PT = 512;                 // threads per CTA (128 registers each: 
 constexpr int TILE = 128;               // pairs a warp advances at a time: a quad of consecutive pairs per lane
 constexpr int EV_BUF = 192;             // quads a warp keeps for the pair-by-pair advance
 constexpr int SPK_BUF = 1024;           // spikes of one CTA and epoch buffered for the listing warps
-constexpr int IN_BUF = 2048;            // input pairs of one CTA with their kick thresholds in shared memory
+constexpr int IN_BUF = 2048;            // input pairs of one CTA with their kick thresholds in shared memory, at least
 constexpr long long BARRIER_TIMEOUT_CYCLES = 8000000000LL;   // ~4 s at 1.9 GHz
 constexpr int MAX_EPOCH = 6;            // steps per epoch at most
 constexpr int K_BITS = 18;              // bits of a local pair index (per < 2^18)
@@ -58,7 +58,9 @@ struct PersistPlan {
     int32_t n_groups = 1;
     int32_t ctas = 0;
     int64_t per = 0;          // pairs per CTA (multiple of 16)
+    int32_t inputs = IN_BUF;  // input pairs of a CTA held in shared memory
     size_t smem = 0;
+    size_t smem_max = 0;      // ... that a block can have
     int32_t launches_per_run = 0;
 };
 
@@ -154,16 +156,17 @@ __device__ __forceinline__ bool grid_wait(const PersistArgs& A, unsigned int tar
 // Shared-memory layout of one CTA (bytes), for `per` pairs.
 struct PersistSmem {
     int32_t v, g, ref, kick, special, events, inputs, spk, hash, ticks, misc, total;
+    int32_t n_inputs;
     PersistSmem() = default;
-    explicit PersistSmem(int32_t per)
+    explicit PersistSmem(int32_t per, int32_t n_in = IN_BUF) : n_inputs(n_in)
     {
         const int32_t per4 = (per + 3) / 4;  // quads
         v = 0;
         g = v + per * 4;
         kick = g + per * 4;                  // two words per quad (epoch parity): bit 4 s + j = kick of pair j at step s
-        inputs = kick + 2 * per4 * 4;        // IN_BUF inputs {local pair | instance << 18, threshold}
+        inputs = kick + 2 * per4 * 4;        // n_inputs inputs {local pair | instance << 18, threshold}
         inputs = (inputs + 15) / 16 * 16;
-        spk = inputs + 8 * IN_BUF;           // two buffers (epoch parity) of SPK_BUF spikes {local pair | step << 18}
+        spk = inputs + 8 * n_inputs;         // two buffers (epoch parity) of SPK_BUF spikes {local pair | step << 18}
         hash = spk + 2 * 4 * SPK_BUF;        // kick hash seeds of (step, instance); per instance the pair-number offset
         ticks = hash + 4 * (MAX_EPOCH + 1) * 64; // reset and stop ticks of up to 64 instances; active steps (epoch parity)
         misc = ticks + 2 * 64 * 8 + 2 * 64 * 4;  // counters
@@ -395,7 +398,7 @@ __device__ __noinline__ void draw_kicks(const PersistParams& P, int32_t s0, int 
     const uint32_t* s_off = s_hash + MAX_EPOCH * 64;
     const int2* s_in = smem_at<int2>(P.lay.inputs);
     const int32_t e0 = P.A.ext_off[blockIdx.x], e1 = P.A.ext_off[blockIdx.x + 1];
-    const int32_t n_in = RASTER ? 0 : min(e1 - e0, IN_BUF);
+    const int32_t n_in = RASTER ? 0 : min(e1 - e0, P.lay.n_inputs);
     for (int32_t e = tid; e < n_in; e += PT) {
         const int2 en = s_in[e];
         const int32_t k = en.x & 0x3ffff, bl = en.x >> 18, na = act[bl];
@@ -727,7 +730,7 @@ __device__ __noinline__ void load_state(const PersistParams& P, int32_t cnt)
         const int32_t k = en.x & 0x3ffff, bi = en.x >> 18;
         const int64_t at = (int64_t)(b0 + bi) * S.n_ext + en.y;
         if (bi < G && S.bias_ext[at] != 0.0f) sr[k] |= 0x80;
-        if (!RASTER && e - e0 < IN_BUF) s_in[e - e0] = make_int2(en.x, bi < G ? kick_threshold(S.p_ext[at]) : 0);
+        if (!RASTER && e - e0 < P.lay.n_inputs) s_in[e - e0] = make_int2(en.x, bi < G ? kick_threshold(S.p_ext[at]) : 0);
     }
     __syncthreads();
     for (int32_t k = 4 * tid; k < cnt; k += 4 * PT)
@@ -908,9 +911,21 @@ inline PersistPlan plan_persistent(int64_t n, int64_t n_pad, int32_t B, bool f64
     P.ctas = ctas;
     P.per = per;
     P.smem = (size_t)PersistSmem((int32_t)per).total;
+    P.smem_max = (size_t)smem_optin;
     P.launches_per_run = n_groups;
     (void)n;
     return P;
+}
+
+// Room for the `most` input pairs that a CTA has, as far as shared memory goes (an even number: what follows is
+// aligned to 16 bytes). Beyond it a kick draws its threshold from two dependent global loads: an epoch's kicks of
+// 5,400 inputs per CTA took 5.0 us with 2,048 of them in shared memory and 2.8 with all (16 x 50,000, all
+// driven at 100 Hz: 2.41 ms per 166 steps and 1.83 with K = 1, 1.16 and 0.99 with K = 6).
+inline void plan_inputs(PersistPlan& P, int32_t most)
+{
+    const int32_t spare = (int32_t)(P.smem_max - (size_t)PersistSmem((int32_t)P.per).total) / 8;
+    P.inputs = std::min((std::max(most, IN_BUF) + 1) & ~1, (IN_BUF + spare) & ~1);
+    P.smem = (size_t)PersistSmem((int32_t)P.per, P.inputs).total;
 }
 
 // Steps per epoch. Longer epochs mean fewer barriers, but the 2K accumulator slots of the group are to stay
@@ -937,7 +952,7 @@ cudaError_t launch_persist_one(const PersistPlan& P, const DevNet& N, const DevS
                                cudaStream_t st)
 {
     auto kern = k_persist<AccT, RASTER, PLASTIC, RECORD, KB>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_max);
     if (e != cudaSuccess) return e;
     for (int32_t q = 0; q < P.n_groups; q++) {
         const int32_t b0 = q * P.group;
@@ -954,7 +969,7 @@ cudaError_t launch_persist_one(const PersistPlan& P, const DevNet& N, const DevS
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, kern, PersistParams{N, S, A, PersistSmem((int32_t)P.per), b0, G, q, (int32_t)P.per});
+        e = cudaLaunchKernelEx(&cfg, kern, PersistParams{N, S, A, PersistSmem((int32_t)P.per, P.inputs), b0, G, q, (int32_t)P.per});
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

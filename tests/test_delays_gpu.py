@@ -70,3 +70,14 @@ def test_engines_in_turn_at_short_delays(torch, n_delay):  # noqa: F811
         gb.set_schedule("step" if k % 2 else "persistent")
         _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps))
     gb.check()
+
+
+@pytest.mark.parametrize("n_delay", [5, 18])
+def test_more_inputs_than_shared_memory_has_room_for(torch, n_delay):  # noqa: F811
+    """Nearly as many pairs as the chip holds, all of them inputs: most thresholds stay in global memory."""
+    gb, eo = _pair(torch, 39_990, 62, n_delay * 0.1, degree=2, driven=1.0, hz=300.0)
+    info = gb.info()
+    assert info.group == 62 and 62 * 39_990 / info.ctas > 16_000
+    for steps in (7, 9):
+        _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps))
+    gb.check()
