@@ -9,14 +9,16 @@
 //               weight pw enters as the Q32.32 delta q32(pw) - q32(w0), pushed at spike time.
 //   state       v[B][n], g[B][n] (f32 or f64), ref[B][n] i8
 //   inputs      ext_idx[n] i32, p_ext[B][n_ext] f32, bias_ext[B][n_ext] f32
-//   delay line  acc[S][B][n_pad] (i32 or i64): synaptic input of the next S ticks (slot = tick mod
-//               S, S = 2 x the persistent engine's epoch, at least 2), rows padded to 16 entries
-//               so that every row starts on a 16-byte boundary at any accumulator width;
-//               items[R][n_groups][cap_c] int2: spike work lists of the last R = n_delay + K steps (K: the
-//               persistent engine's epoch, 1 without it; a list is emptied K steps before it is filled
-//               again), one per instance group; item_count[R][n_groups];
-//               pring[R_pl][B][n_ppost] i64: plastic input (R_pl = n_delay + K: a slot
-//               is cleared by its reader at least one epoch before anyone pushes into it again);
+//   delay line  acc[S][B][n_pad] (i16, i32 or i64): synaptic input of the next S ticks (slot = tick mod
+//               S, S = 2 x the persistent engine's epoch, at least 2; 2 in the step engine's own array where
+//               the persistent engine's is 16 bits wide), rows padded to 16 entries so that every row
+//               starts on a 16-byte boundary at any accumulator width;
+//               items[R][n_groups][cap_c] int2: spike work lists of the last R = n_delay + 1 steps, one per
+//               instance group (a list is overwritten after its arrivals were pushed);
+//               item_count[R_pl][n_groups], R_pl = n_delay + K (K: the persistent engine's epoch, 1
+//               without it): a count is zeroed K steps before its list is filled again;
+//               pring[R_pl][B][n_ppost] i64: plastic input (a slot is cleared by its reader at least
+//               one epoch before anyone pushes into it again);
 //               with pull propagation also masks[R][n][ceil(B/64)] u64: which instances each
 //               neuron spiked in, and the connectome by postsynaptic neuron (colptr, cpre, ccnt/cwfx)
 //
@@ -35,7 +37,7 @@ namespace fb {
 struct DevNet {
     int64_t n, n_pad;
     int32_t B, n_delay, R, n_ref;
-    int32_t R_pl;              // plastic input ring slots: n_delay + the persistent engine's epoch
+    int32_t R_pl;              // slots of the plastic input and of the list lengths: n_delay + the persistent engine's epoch
     const int64_t* rowptr;
     const int32_t* col;
     const int16_t* cnt;
@@ -67,7 +69,7 @@ struct DevState {
     int32_t n_slots;
     int64_t* pring;
     int2* items;               // [R][n_groups][cap_c]
-    int32_t* item_count;       // [R][n_groups]
+    int32_t* item_count;       // [R_pl][n_groups]
     int64_t cap_c;             // items per (step, group) list
     int32_t group;             // instances per group (group of instance b = b / group)
     int32_t n_groups;
@@ -108,13 +110,14 @@ template <typename Real> __device__ __forceinline__ const Lif<Real>& lif_of(cons
 template <> __device__ __forceinline__ const Lif<float>& lif_of<float>(const DevNet& N) { return N.L32; }
 template <> __device__ __forceinline__ const Lif<double>& lif_of<double>(const DevNet& N) { return N.L64; }
 
-__device__ __forceinline__ int2* list_of(const DevState& S, int64_t slot, int32_t q)
+// the work list of step t and group q, and its length
+__device__ __forceinline__ int2* list_of(const DevNet& N, const DevState& S, int64_t t, int32_t q)
 {
-    return S.items + ((int64_t)slot * S.n_groups + q) * S.cap_c;
+    return S.items + (pos_mod(t, N.R) * S.n_groups + q) * S.cap_c;
 }
-__device__ __forceinline__ int32_t* count_of(const DevState& S, int64_t slot, int32_t q)
+__device__ __forceinline__ int32_t* count_of(const DevNet& N, const DevState& S, int64_t t, int32_t q)
 {
-    return S.item_count + (int64_t)slot * S.n_groups + q;
+    return S.item_count + pos_mod(t, N.R_pl) * S.n_groups + q;
 }
 
 // Fire-and-forget reductions into global memory (no value comes back; the address is converted to
@@ -141,7 +144,7 @@ __device__ __forceinline__ int2 make_item(const DevNet& N, int32_t i, int32_t b,
 
 // Append `nch` work items (this lane's spike: chunks 0..nch-1 of row i of instance b) to the list of
 // the lane's group; one atomic per warp and list (the ballot/shuffle compaction).
-__device__ __forceinline__ void warp_append(const DevNet& N, const DevState& S, int64_t slot, int nch, int32_t i,
+__device__ __forceinline__ void warp_append(const DevNet& N, const DevState& S, int64_t t, int nch, int32_t i,
                                             int32_t b)
 {
     const unsigned FULL = 0xffffffffu;
@@ -161,10 +164,10 @@ __device__ __forceinline__ void warp_append(const DevNet& N, const DevState& S, 
         }
         const int total = __shfl_sync(FULL, incl, 31);
         int base = 0;
-        if (lane == 31) base = atomicAdd(count_of(S, slot, kk), total);
+        if (lane == 31) base = atomicAdd(count_of(N, S, t, kk), total);
         base = __shfl_sync(FULL, base, 31);
         if (mine) {
-            int2* list = list_of(S, slot, kk);
+            int2* list = list_of(N, S, t, kk);
             const int64_t start = (int64_t)base + incl - nch;
             for (int ch = 0; ch < nch; ch++) {
                 const int64_t p = start + ch;
@@ -249,7 +252,6 @@ __device__ __forceinline__ void update_pair(const DevNet& N, const DevState& S, 
 {
     const int64_t n = N.n, t = A.t;
     const Lif<Real>& L = lif_of<Real>(N);
-    const int64_t slot = pos_mod(t, N.R);
     const int32_t i = (int32_t)i64;
     int nch = 0;
     if (i64 < n && t < S.stop_tick[b]) {
@@ -280,7 +282,7 @@ __device__ __forceinline__ void update_pair(const DevNet& N, const DevState& S, 
         if (r != r0) S.ref[pair] = (int8_t)r;
         if (spk) {
             A.counts[pair] += 1;
-            if (S.masks) atomicOr(S.masks + (slot * n + i) * S.mask_words + (b >> 6), 1ull << (b & 63));
+            if (S.masks) atomicOr(S.masks + (pos_mod(t, N.R) * n + i) * S.mask_words + (b >> 6), 1ull << (b & 63));
             const int64_t len = N.rowptr[i + 1] - N.rowptr[i];
             nch = (int)((len + CHUNK - 1) / CHUNK);
             if (PLASTIC) push_plastic_row(N, S, t, b, i);
@@ -292,7 +294,7 @@ __device__ __forceinline__ void update_pair(const DevNet& N, const DevState& S, 
             }
         }
     }
-    warp_append(N, S, slot, nch, i, b);
+    warp_append(N, S, t, nch, i, b);
 }
 
 // 8 consecutive CSR entries of one lane: weights (one or four 16-byte loads) and columns (two).
@@ -349,13 +351,13 @@ __device__ __forceinline__ void push_item(const DevNet& N, AccT* acc_b, int64_t 
     }
 }
 
-// Items of list (slot, q): its count, clamped to the capacity (L2: other SMs appended to it)
-__device__ __forceinline__ int32_t list_length(const DevState& S, int64_t slot, int32_t q)
+// Items of the list of step t and group q: its count, clamped to the capacity (L2: other SMs appended to it)
+__device__ __forceinline__ int32_t list_length(const DevNet& N, const DevState& S, int64_t t, int32_t q)
 {
-    return (int32_t)min((int64_t)max(__ldcg(count_of(S, slot, q)), 0), S.cap_c);
+    return (int32_t)min((int64_t)max(__ldcg(count_of(N, S, t, q)), 0), S.cap_c);
 }
 
-// Scatter the items [g0, g1) of list (slot of spike step s = t+1-n_delay, group q) into acc_next; lane
+// Scatter the items [g0, g1) of the list of spike step s = t+1-n_delay and group q into acc_next; lane
 // group `lg` of `n_lg` (LANES lanes each, lane `lane` within it) takes items g0+lg, g0+lg+n_lg, ...
 // Items of instance b are skipped unless reset_tick[b] <= s and t+1 < stop_tick[b].
 template <typename AccT, int LANES>
@@ -363,7 +365,7 @@ __device__ __forceinline__ void push_range(const DevNet& N, const DevState& S, i
                                            int64_t g0, int64_t g1, int64_t lg, int64_t n_lg, int lane)
 {
     const int64_t s = t + 1 - N.n_delay;
-    const int2* list = list_of(S, pos_mod(s, N.R), q);
+    const int2* list = list_of(N, S, s, q);
     for (int64_t g = g0 + lg; g < g1; g += n_lg) {
         const int2 item = __ldcg(list + g);
         const int32_t b = item.y >> CHUNK_BITS;
@@ -390,10 +392,9 @@ template <typename AccT>
 __device__ __forceinline__ void push_lists(const DevNet& N, const DevState& S, int64_t t, int lanes, int blk, int n_blk)
 {
     AccT* acc = acc_slot<AccT>(N, S, t + 1);
-    const int64_t slot = pos_mod(t + 1 - N.n_delay, N.R);
     __shared__ int32_t s_total;
     for (int32_t q = 0; q < S.n_groups; q++) {
-        if (threadIdx.x == 0) s_total = list_length(S, slot, q);     // (one load per block: they all hit one address)
+        if (threadIdx.x == 0) s_total = list_length(N, S, t + 1 - N.n_delay, q);     // (one load per block: they all hit one address)
         __syncthreads();
         const int64_t total = s_total;
         const int64_t g0 = total * blk / n_blk, g1 = total * (blk + 1) / n_blk;
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(256) k_step(const __grid_constant__ DevNet N, 
     const uint32_t u = blockIdx.x - (uint32_t)G.n_push;
     const int32_t b = (int32_t)(u / (uint32_t)G.per);
     if (u == 0)                // the lists consumed by the push at t-1 start empty again
-        for (int32_t k = threadIdx.x; k < S.n_groups; k += blockDim.x) *count_of(S, pos_mod(A.t - N.n_delay, N.R), k) = 0;
+        for (int32_t k = threadIdx.x; k < S.n_groups; k += blockDim.x) *count_of(N, S, A.t - N.n_delay, k) = 0;
     const int64_t i0 = (int64_t)(u % (uint32_t)G.per) * G.tiles * 256 + threadIdx.x;
 #pragma unroll 1
     for (int k = 0; k < G.tiles; k++) update_pair<Real, AccT, RASTER, PLASTIC, RECORD>(N, S, A, b, i0 + k * 256);

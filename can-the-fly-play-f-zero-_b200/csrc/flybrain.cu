@@ -115,8 +115,7 @@ __global__ void k_largest(unsigned long long* sums, int64_t n)
         atomicMax(sums + n, sums[i]);
 }
 
-// The accumulators from 32 to 16 bits (two pairs to a word) or back, when a run starts on the other engine;
-// those left behind are zero
+// One slot of accumulators from 32 to 16 bits (two pairs to a word) or back
 __global__ void k_repack(int32_t* wide, int32_t* narrow, int64_t words, bool to_narrow)
 {
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (int64_t)gridDim.x * blockDim.x) {
@@ -124,11 +123,9 @@ __global__ void k_repack(int32_t* wide, int32_t* narrow, int64_t words, bool to_
         if (to_narrow) {
             const int2 x = *p;
             narrow[w] = (int32_t)(((uint32_t)x.y << 16) + (uint32_t)x.x);
-            if (x.x | x.y) *p = make_int2(0, 0);
         } else {
             const int32_t x = narrow[w];
             *p = make_int2(lo16(x), hi16(x));
-            if (x) narrow[w] = 0;
         }
     }
 }
@@ -194,9 +191,9 @@ struct fb_brain {
     PlasticPlan plastic;              // current plastic plan
     // delay line
     void* acc = nullptr;          // [n_slots][B][n_pad] int32 or int64
-    void* acc16 = nullptr;        // the same in 16 bits for the persistent engine, where every input sum fits
+    void* acc16 = nullptr;        // [n_slots16][B][n_pad] int16 for the persistent engine, where every input sum fits
     bool live16 = false;          // the input in flight is in acc16 (acc is zero), else in acc (acc16 is zero)
-    int32_t n_slots = 2;
+    int32_t n_slots = 2, n_slots16 = 0;
     EpochPlan epochs;             // persistent engine: steps between grid barriers
     int32_t last_epoch = 1;       // ... of the last run (before the first: with late listing)
     int64_t pushed_until = 1;     // the arrivals of every tick < pushed_until are in acc
@@ -253,7 +250,7 @@ struct fb_brain {
     {
         DevState S{};
         S.v = v; S.g = g; S.ref = ref; S.pw = pw; S.ext_idx = ext_idx; S.n_ext = (int32_t)n_ext;
-        S.p_ext = p_ext; S.bias_ext = bias_ext; S.acc = live16 ? acc16 : acc; S.n_slots = n_slots; S.pring = pring;
+        S.p_ext = p_ext; S.bias_ext = bias_ext; S.acc = live16 ? acc16 : acc; S.n_slots = live16 ? n_slots16 : n_slots; S.pring = pring;
         S.items = items; S.item_count = item_count; S.cap_c = cap_c; S.group = list_group;
         S.n_groups = n_groups; S.reset_tick = reset_tick;
         S.stop_tick = stop_tick; S.err = err_d; S.seed = seed;
@@ -479,13 +476,14 @@ extern "C" int fb_create(const fb_params* P, const int64_t* indptr, const int32_
     const bool narrow = h->plan.group > 0 && h->acc_mode == 0 && largest <= INT16_MAX;
     if (h->plan.group > 0) h->epochs = plan_epochs(h->n_delay, narrow ? 2 : (int)ab);
     h->last_epoch = h->epochs.late;
-    h->n_slots = 2 * h->epochs.steps;
-    h->R_pl = h->R = h->n_delay + h->epochs.steps;
+    (narrow ? h->n_slots16 : h->n_slots) = 2 * h->epochs.steps;      // (the step engine needs two)
+    h->R = h->n_delay + 1;
+    h->R_pl = h->n_delay + h->epochs.steps;
     TRY(dalloc((char**)&h->acc, nbp * ab * h->n_slots, tb));
     CU(cudaMemset(h->acc, 0, nbp * ab * h->n_slots));
     if (narrow) {
-        TRY(dalloc((char**)&h->acc16, nbp * 2 * h->n_slots, tb));
-        CU(cudaMemset(h->acc16, 0, nbp * 2 * h->n_slots));
+        TRY(dalloc((char**)&h->acc16, nbp * 2 * h->n_slots16, tb));
+        CU(cudaMemset(h->acc16, 0, nbp * 2 * h->n_slots16));
         h->live16 = true;             // (all zero: nothing to carry over)
     }
     h->list_group = h->plan.group > 0 ? h->plan.group : h->B;
@@ -496,7 +494,7 @@ extern "C" int fb_create(const fb_params* P, const int64_t* indptr, const int32_
     h->cap_c = segment_capacity(H, h->n_pad, h->list_group, (int64_t)h->list_group * h->n_pad, 1);
     h->cap_alloc = h->cap_c;
     TRY(dalloc(&h->items, (size_t)h->R * h->n_groups * h->cap_c, tb));
-    TRY(dalloc(&h->item_count, (size_t)h->R * h->n_groups, tb));
+    TRY(dalloc(&h->item_count, (size_t)h->R_pl * h->n_groups, tb));
     TRY(dalloc(&h->reset_tick, (size_t)batch, tb));
     TRY(dalloc(&h->stop_tick, (size_t)batch, tb));
     TRY(dalloc(&h->fly_mask, (size_t)batch, tb));
@@ -630,7 +628,8 @@ extern "C" int fb_reset(fb_brain* h, const int32_t* flies, int32_t n_flies, void
         k_reset<double><<<blocks, 256, 0, st>>>((double*)h->v, (double*)h->g, h->ref, h->acc, h->n_slots, ab, h->pring,
                                                 h->R_pl, h->B, h->n, h->n_pad, h->n_ppost, mask, h->params.v_rest);
     else
-        k_reset<float><<<blocks, 256, 0, st>>>((float*)h->v, (float*)h->g, h->ref, h->live16 ? h->acc16 : h->acc, h->n_slots, ab, h->pring,
+        k_reset<float><<<blocks, 256, 0, st>>>((float*)h->v, (float*)h->g, h->ref, h->live16 ? h->acc16 : h->acc,
+                                               h->live16 ? h->n_slots16 : h->n_slots, ab, h->pring,
                                                h->R_pl, h->B, h->n, h->n_pad, h->n_ppost, mask, (float)h->params.v_rest);
     CU(cudaGetLastError());
     h->launches += 1;
@@ -642,7 +641,7 @@ extern "C" int fb_reset(fb_brain* h, const int32_t* flies, int32_t n_flies, void
             h->mask_from = 0;
             h->masks_dirty = false;
         }
-        CU(cudaMemsetAsync(h->item_count, 0, (size_t)h->R * h->n_groups * sizeof(int32_t), st));
+        CU(cudaMemsetAsync(h->item_count, 0, (size_t)h->R_pl * h->n_groups * sizeof(int32_t), st));
     }
     k_set_ticks<<<(h->B + 255) / 256, 256, 0, st>>>(h->reset_tick, mask, h->B, h->t);
     CU(cudaGetLastError());
@@ -984,11 +983,17 @@ extern "C" int fb_run(fb_brain* h, int32_t steps, int32_t* counts_out, const uin
     if (engine == FB_ENGINE_AUTO)
         engine = (h->plan.group > 0 && !h->f64 && h->prop == FB_PROP_PUSH) ? FB_ENGINE_PERSISTENT : FB_ENGINE_STEP;
     const bool persistent = engine == FB_ENGINE_PERSISTENT && h->plan.group > 0 && !h->f64;
-    if (h->acc16 && h->live16 != persistent) {                // the input in flight follows the engine
-        const int64_t accs = (int64_t)h->n_slots * h->B * h->n_pad / 2;
-        k_repack<<<(unsigned)std::min<int64_t>((accs + 255) / 256, (int64_t)h->sm_count * 16), 256, 0, st>>>(
-            (int32_t*)h->acc, (int32_t*)h->acc16, accs, persistent);
+    if (h->acc16 && h->live16 != persistent) {
+        // the input in flight follows the engine: between runs that is what arrives at tick t; the array that
+        // is left is zeroed (an instance whose stop was moved before t has input there that nobody took)
+        const int64_t pairs = (int64_t)h->B * h->n_pad;
+        int32_t* wide = (int32_t*)h->acc + h->t % h->n_slots * pairs;
+        int32_t* half = (int32_t*)h->acc16 + h->t % h->n_slots16 * (pairs / 2);
+        k_repack<<<(unsigned)std::min<int64_t>((pairs / 2 + 255) / 256, (int64_t)h->sm_count * 16), 256, 0, st>>>(wide, half, pairs / 2,
+                                                                                                              persistent);
         CU(cudaGetLastError());
+        if (persistent) CU(cudaMemsetAsync(h->acc, 0, (size_t)pairs * 4 * h->n_slots, st));
+        else CU(cudaMemsetAsync(h->acc16, 0, (size_t)pairs * 2 * h->n_slots16, st));
         h->launches += 1;
         h->live16 = persistent;
     }

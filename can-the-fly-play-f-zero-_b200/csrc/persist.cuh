@@ -291,7 +291,7 @@ __device__ __forceinline__ void list_one(const PersistParams& P, int32_t k, int3
 // Its work items at `base`, .. of its step's list
 __device__ __forceinline__ void write_items(const PersistParams& P, int64_t t, int32_t base, int64_t r0, int64_t r1, int32_t b)
 {
-    int2* list = list_of(P.S, pos_mod(t, P.N.R), P.q);
+    int2* list = list_of(P.N, P.S, t, P.q);
     for (int64_t r = r0; r < r1; r += CHUNK, base++) {
         if (base < P.S.cap_c) list[base] = make_int2((int32_t)r, (b << CHUNK_BITS) | (int32_t)min((int64_t)CHUNK, r1 - r));
         else atomicExch(P.S.err, 1);
@@ -308,7 +308,7 @@ __device__ __noinline__ void list_overflow(const PersistParams& P, int32_t k, in
     list_one<PLASTIC, RECORD>(P, k, s, r0, r1, b);
     const int64_t t = P.A.t0 + s;
     const int nch = row_items(r0, r1);
-    if (nch) write_items(P, t, atomicAdd(count_of(P.S, pos_mod(t, P.N.R), P.q), nch), r0, r1, b);
+    if (nch) write_items(P, t, atomicAdd(count_of(P.N, P.S, t, P.q), nch), r0, r1, b);
 }
 
 // The spikes of local pair k (bit 4 s: at step s of the epoch whose first step is s0) into the buffer of
@@ -355,7 +355,7 @@ __device__ __noinline__ void list_epoch(const PersistParams& P, int par, int32_t
         if (tid0 < kc) {
             const int32_t n = C->cursor[tid0];
             C->cursor[tid0] = 0;
-            C->base[tid0] = n ? atomicAdd(count_of(P.S, pos_mod(P.A.t0 + s0 + tid0, P.N.R), P.q), n) : 0;
+            C->base[tid0] = n ? atomicAdd(count_of(P.N, P.S, P.A.t0 + s0 + tid0, P.q), n) : 0;
         }
         sync();
         if (r1 > r0) write_items(P, P.A.t0 + s0 + ds, C->base[ds] + at, r0, r1, b);
@@ -450,7 +450,7 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
     // this CTA's share of each list, flattened
     int32_t from = 0, len_k = 0;
     if (lane < nl && a0 + lane >= N.n_delay) {
-        const int64_t total = list_length(S, pos_mod(a0 + lane - N.n_delay, N.R), P.q);
+        const int64_t total = list_length(N, S, a0 + lane - N.n_delay, P.q);
         from = (int32_t)(total * blockIdx.x / gridDim.x);
         len_k = (int32_t)(total * (blockIdx.x + 1) / gridDim.x) - from;
     }
@@ -477,7 +477,7 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
             for (int u = 1; u < MAX_EPOCH; u++)
                 if (off[u] <= j) { k = u; g = first[u] + (j - off[u]); }
             const int32_t ls = list0 + k < N.R ? list0 + k : list0 + k - N.R;
-            const int2 item = __ldcg(list_of(S, ls, P.q) + g);
+            const int2 item = __ldcg(S.items + ((int64_t)ls * S.n_groups + P.q) * S.cap_c + g);
             const int32_t bl = (item.y >> CHUNK_BITS) - P.b0;
             start = item.x;
             if (a0 + k - N.n_delay >= s_reset[bl] && a0 + k < s_stop[bl]) len = item.y & ((1 << CHUNK_BITS) - 1);
@@ -806,9 +806,9 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
         if (is_l) {
             const int32_t kc = min(K, A.steps - ep0);
             if (A.list_late && ep0 > 0) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, K, false);
-            // the lists whose items arrive in this epoch were pushed before it: they are empty when they are
-            // filled again, K steps after the ticks of this epoch
-            if (blockIdx.x == 0 && tid < kc) *count_of(P.S, pos_mod(A.t0 + ep0 + tid - P.N.n_delay, P.N.R), P.q) = 0;
+            // the lists whose items arrive in this epoch were pushed before it: their lengths are zero when the
+            // slots serve again, K steps after the ticks of this epoch
+            if (blockIdx.x == 0 && tid < kc) *count_of(P.N, P.S, A.t0 + ep0 + tid - P.N.n_delay, P.q) = 0;
             if (ep0 + kc < A.steps) prepare_epoch<RASTER>(P, ep0 + kc, min(K, A.steps - ep0 - kc), par ^ 1, tid, LIST_THREADS);
             if (tid == 0) {
                 C->tile[par ^ 1] = 0;

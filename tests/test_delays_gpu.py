@@ -81,3 +81,42 @@ def test_more_inputs_than_shared_memory_has_room_for(torch, n_delay):  # noqa: F
     for steps in (7, 9):
         _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps))
     gb.check()
+
+
+@pytest.mark.parametrize("n_delay", [3, 5, 18])
+def test_stops_on_one_engine_then_the_other(torch, n_delay):  # noqa: F811
+    """Instances that stop (one with input still on its way) while one engine runs, then the other takes over: what
+    is in flight follows, what a stopped instance left behind does not come back after its reset."""
+    gb, eo = _pair(torch, 1201, 6, n_delay * 0.1, plastic=0.05, bias=0.03)
+
+    def run(engine, steps, stop=None):
+        gb.set_schedule(engine)
+        _same(gb, eo, gb.run_steps(steps), eo.run_steps(steps) if stop is None else eo.run_steps(steps, stop_tick=stop))
+
+    for first, second in (("step", "persistent"), ("persistent", "step"), ("step", "persistent")):
+        run(first, 25)
+        left = np.array([0, 1, 4, 9, 17, -1])                      # instance 0 stops with the next tick's input pushed
+        gb.set_run_length(left)
+        stop = np.where(left < 0, 2 ** 62, eo.t + left).astype(np.int64)
+        run(first, 11, stop)
+        run(second, 13, stop)
+        run(first, 2, stop)
+        ended = [0, 1, 2, 3, 4]
+        gb.reset(ended)
+        eo.reset_flies(ended)
+        gb.set_run_length(np.full(6, -1))
+        run(second, 27)
+    gb.check()
+
+
+def test_device_memory_of_a_count_network(torch):  # noqa: F811
+    """The delay line's bytes for 16-bit sums: 12 slots of 2 and 2 of 4 per pair, n_delay + 1 lists of every pair."""
+    from flyzero_b200.brain import LIFParams
+    from flyzero_b200.gpu import BatchBrain
+    from test_epochs_gpu import _net
+
+    n, B = 20_000, 8
+    w = _net(n, 8, 1, True)
+    a, b = (BatchBrain(w, LIFParams(), batch=B * k).info() for k in (1, 2))
+    pair = 9 + 4 + 12 * 2 + 2 * 4 + 19 * 8             # state, ext_idx aside; a row is one item
+    assert b.epoch == 6 and b.bytes_device - a.bytes_device <= 1.02 * B * n * pair
