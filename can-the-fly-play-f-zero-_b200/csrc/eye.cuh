@@ -3,8 +3,9 @@
 // frames are already on the device, so no rates cross the bus and no host loop runs per frame.
 //
 // The default is two launches: k_eye_grid (a thread per instance and grid cell: luminance, high-pass,
-// delay arms, colours) and k_eye_neurons (several blocks per instance, its grids in shared memory). Grids
-// too large for that take four grid-wide kernels, which state the steps one by one:
+// delay arms, colours) and k_eye_neurons (several blocks per instance, its grids in shared memory); small eyes
+// take k_eye_neurons alone, one block per instance, which forms the grids itself. Grids too large for
+// shared memory take four grid-wide kernels, which state the steps one by one:
 //   k_eye_cells    one thread per (instance, grid cell):
 //                  lum = mean over the cell x cell block of mean(R, G, B) / 255 (vision.py:136-140),
 //                  each block row summed with NumPy's pairwise rule, the row sums added in order;
@@ -43,7 +44,7 @@ struct EyeArgs {
     double gain, sustained;
     const uint8_t* frames;      // (B, H, W, 3)
     const uint8_t* flip;        // (B) mirror the frame left-right, or nullptr
-    uint8_t* restart;           // (B) start the filters from this frame; cleared by k_eye_delay
+    uint8_t* restart;           // (B) start the filters from this frame; cleared when it is done
     float* lum;                 // (B, gh, gw)
     float* lp;                  // (B, gh, gw)
     float* sig;                 // (B, 2, gh, gw)  ON, OFF
@@ -225,13 +226,13 @@ __global__ void k_eye_delay(const EyeArgs a)
     if (p % (2 * cells) == 0) a.restart[p / (2 * cells)] = 0;
 }
 
-// ---- the same eye in two launches (the default) ----------------------------------------------------------
+// ---- the same eye in two launches or one (the default) ---------------------------------------------------
 // The grid of every instance by one thread per cell, then the neurons of an instance by several blocks.
-// One block per instance (its grid in shared memory) kept 64 instances on 64 of the 148 SMs and waited
-// through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16.5,
+// One block per instance for all of it (its grid in shared memory) kept 64 instances on 64 of the 148 SMs and
+// waited through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16.5,
 // 22.0 together as a dependent chain whose second kernel reads its tables beside the first (23.3 without
-// that, 26.6 as ordinary launches). Small eyes lose a little by the second launch: 30 of 1,000 cells and 3,287
-// neurons 12.0 us a call against 10.8.
+// that, 26.6 as ordinary launches). Small eyes, and as many as there are SMs, lose more by the second launch
+// than they gain: they take one block per instance again (fb_motion_eye says where the line lies).
 
 // x / 3 and x / 255 rounded to nearest for the values a pixel can take (R + G + B and its third, a byte): one
 // Newton correction of the quotient by its exact remainder (Markstein 1990). Checked against the
@@ -303,9 +304,47 @@ __device__ __forceinline__ void cell_sums(const EyeArgs& a, const uint8_t* fr, b
     }
 }
 
-// One thread per (instance, grid cell): luminance, colour grids, high-pass signal (`sig`, the ON half of
-// the state: hp itself; ON is max(hp, 0), OFF max(-hp, 0)) and the delay arms: this frame's into the
-// scratch halves (ON: sig's OFF half; OFF: the integral image's place) and the next frame's into dly.
+// One grid cell q of instance b (p = b * cells + q): luminance, colours (when chromatic), high-pass signal (hp itself; ON is
+// max(hp, 0), OFF max(-hp, 0)) and this frame's delay arms; the filters go on to the next frame's.
+struct EyeCell {
+    float lum, blue, green, hp, on, off;
+};
+template <bool VEC4>
+__device__ __forceinline__ EyeCell eye_cell(const EyeArgs& a, int32_t b, int32_t q, int64_t p, bool restart, bool fl)
+{
+    const int32_t y = q / a.gw, x = q - y * a.gw;
+    const int64_t cells = (int64_t)a.gh * a.gw;
+    float* dly = a.dly + (int64_t)b * 2 * cells + q;
+    EyeCell c;
+    float lp, s, sb, sg;
+    auto filters = [&]() {
+        lp = a.lp[p];
+        c.on = dly[0];
+        c.off = dly[cells];
+    };
+    if (VEC4) filters();                                           // (in flight beside the pixels)
+    cell_sums<VEC4>(a, a.frames + (int64_t)b * a.H * a.W * 3, fl, y, x, a.chromatic != 0, s, sb, sg);
+    if (!VEC4) filters();                                          // (beside cells of any size they were spilled)
+    const float area = (float)(a.cell * a.cell);
+    c.lum = __fdiv_rn(s, area);
+    if (a.chromatic) {
+        c.blue = __fdiv_rn(sb, area);
+        c.green = __fdiv_rn(sg, area);
+    }
+    if (restart) {
+        lp = c.lum;
+        c.on = c.off = 0.0f;
+    }
+    lp = __fadd_rn(lp, __fmul_rn(a.a_hp, __fsub_rn(c.lum, lp)));
+    a.lp[p] = lp;
+    c.hp = __fsub_rn(c.lum, lp);
+    dly[0] = __fadd_rn(c.on, __fmul_rn(a.a_d, __fsub_rn(fmaxf(c.hp, 0.0f), c.on)));
+    dly[cells] = __fadd_rn(c.off, __fmul_rn(a.a_d, __fsub_rn(fmaxf(-c.hp, 0.0f), c.off)));
+    return c;
+}
+
+// One thread per (instance, grid cell), the results for k_eye_neurons in the scratch arrays (hp: the ON half of
+// `sig`; the delay arms: its OFF half and the integral image's place).
 // Bound by instruction issue: twenty instructions a pixel.
 template <bool VEC4>
 __global__ void __launch_bounds__(256) k_eye_grid(const EyeArgs a)
@@ -315,46 +354,32 @@ __global__ void __launch_bounds__(256) k_eye_grid(const EyeArgs a)
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (int64_t)a.B * cells) return;
     const int32_t b = (int32_t)(p / cells), q = (int32_t)(p - (int64_t)b * cells);
-    const int32_t y = q / a.gw, x = q - y * a.gw;
-    const bool restart = a.restart[b] != 0, fl = a.flip && a.flip[b];
-    float* dly = a.dly + (int64_t)b * 2 * cells + q;
-    float lp = a.lp[p], d_on = dly[0], d_off = dly[cells];          // (in flight beside the pixels)
-    float s, sb, sg;
-    cell_sums<VEC4>(a, a.frames + (int64_t)b * a.H * a.W * 3, fl, y, x, a.chromatic != 0, s, sb, sg);
-    const float area = (float)(a.cell * a.cell);
-    const float lum = __fdiv_rn(s, area);
-    a.lum[p] = lum;
+    const EyeCell c = eye_cell<VEC4>(a, b, q, p, a.restart[b] != 0, a.flip && a.flip[b]);
+    a.lum[p] = c.lum;
     if (a.chromatic) {
-        a.col[(int64_t)b * 2 * cells + q] = __fdiv_rn(sb, area);
-        a.col[((int64_t)b * 2 + 1) * cells + q] = __fdiv_rn(sg, area);
+        a.col[(int64_t)b * 2 * cells + q] = c.blue;
+        a.col[((int64_t)b * 2 + 1) * cells + q] = c.green;
     }
-    if (restart) {
-        lp = lum;
-        d_on = d_off = 0.0f;
-    }
-    lp = __fadd_rn(lp, __fmul_rn(a.a_hp, __fsub_rn(lum, lp)));
-    a.lp[p] = lp;
-    const float hp = __fsub_rn(lum, lp);
-    a.sig[(int64_t)b * 2 * cells + q] = hp;
-    a.sig[((int64_t)b * 2 + 1) * cells + q] = d_on;
-    a.ii[(int64_t)b * (a.gh + 1) * (a.gw + 1) + q] = d_off;
-    dly[0] = __fadd_rn(d_on, __fmul_rn(a.a_d, __fsub_rn(fmaxf(hp, 0.0f), d_on)));
-    dly[cells] = __fadd_rn(d_off, __fmul_rn(a.a_d, __fsub_rn(fmaxf(-hp, 0.0f), d_off)));
+    a.sig[(int64_t)b * 2 * cells + q] = c.hp;
+    a.sig[((int64_t)b * 2 + 1) * cells + q] = c.on;
+    a.ii[(int64_t)b * (a.gh + 1) * (a.gw + 1) + q] = c.off;
 }
 
 // The neurons [blockIdx.x * run, ...) of instance blockIdx.y. The block keeps the instance's grids in shared
 // memory (a neuron gathers up to four cells of them), forms the integral image there (every block of an
-// instance for itself: sharing it would cost a launch), and takes the neurons in chunks sorted by the
-// kind of their channel, so that a warp works on one kind; their rates go out in neuron order through
-// shared memory. Gathered from L1 and unsorted, 64 x 12,246 neurons took 25.7 us, now 16.5; what bounds it is
-// instruction issue (~200 a neuron, 60 of them the sort).
-constexpr int EYE_THREADS = 1024, EYE_UNROLL = 4, EYE_CHUNK = EYE_THREADS * EYE_UNROLL;
+// instance for itself: sharing it would cost a launch), and takes the neurons in chunks. SORT: a chunk's are
+// sorted by the kind of their channel, so that a warp works on one kind, and their rates go out in neuron
+// order through shared memory; without it a thread takes its own. Gathered from L1 and unsorted, 64 x
+// 12,246 neurons took 25.7 us, now 16.5; what bounds it is instruction issue (~200 a neuron, 60 of them
+// the sort, which pays where the contrast's FP64 is long: fb_motion_eye). 64 registers, so one block of
+// 1,024 threads an SM, or two of 512.
+constexpr int EYE_THREADS = 1024, EYE_UNROLL = 4;              // (a chunk's entries are numbered in 12 bits)
 
 constexpr int EYE_SMEM_MAX = 227 * 1024;                          // of a block, all of it dynamic: the kernel has no static arrays
-struct EyeSmem {                                                   // offsets in floats
-    int64_t hp, on, off, lum, ii, col, rate, order, kind, total;
+struct EyeSmem {                                                   // offsets in floats (a grid has at most 1023 x 1023 cells)
+    int32_t hp, on, off, lum, ii, col, rate, order, kind, total;
     EyeSmem() = default;
-    EyeSmem(int64_t cells, int64_t ii_cells, bool sust, bool chrom)
+    EyeSmem(int32_t threads, int32_t cells, int32_t ii_cells, bool sust, bool chrom)
     {
         hp = 0;
         on = hp + cells;
@@ -363,8 +388,8 @@ struct EyeSmem {                                                   // offsets in
         ii = lum + (sust ? cells : 0);
         col = ii + (sust ? ii_cells : 0);
         rate = col + (chrom ? 2 * cells : 0);
-        order = rate + EYE_CHUNK;
-        kind = order + EYE_CHUNK;
+        order = rate + EYE_UNROLL * threads;
+        kind = order + EYE_UNROLL * threads;
         total = kind + 4;
     }
 };
@@ -384,8 +409,12 @@ __device__ __forceinline__ void running_sum(float* v, int32_t n, int32_t stride)
     for (; i < n; i++) v[i * stride] = c = __fadd_rn(c, v[i * stride]);
 }
 
-__global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, const EyeSmem S, int32_t run)
+// where a block's grids come from: k_eye_grid's results, or its own pixels (one block per instance then)
+enum { EYE_GRID_READ = 0, EYE_GRID_OWN = 1, EYE_GRID_OWN4 = 2 };
+template <int GRID, bool SORT, int T>                             // T threads; as a variable it cost 5 %
+__global__ void __launch_bounds__(T, EYE_THREADS / T) k_eye_neurons(const EyeArgs a, const EyeSmem S, int32_t run)
 {
+    constexpr int32_t chunk = EYE_UNROLL * T;
     extern __shared__ float sm[];
     const int32_t b = blockIdx.y, W1 = a.gw + 1, tid = threadIdx.x, lane = tid & 31;
     const int32_t cells = a.gh * a.gw;
@@ -401,7 +430,7 @@ __global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, co
     auto fetch = [&](int32_t first) {
 #pragma unroll
         for (int u = 0; u < EYE_UNROLL; u++) {
-            const int32_t k = first + tid + u * EYE_THREADS;
+            const int32_t k = first + tid + u * T;
             cell[u] = -1;
             chan[u] = slot[u] = 0;
             if (k >= k1) continue;
@@ -411,86 +440,118 @@ __global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, co
             if (x >= 0 && x < a.gw && y >= 0 && y < a.gh && c < EYE_CHANNELS && slot[u] >= 0 && slot[u] < a.n_ext) cell[u] = y * a.gw + x;
         }
     };
-    fetch(blockIdx.x * run);                                       // (the caller's tables: they are older than k_eye_grid)
-    pdl_chain();
+    if (GRID != EYE_GRID_READ) pdl_chain();
+    fetch(blockIdx.x * run);                                       // (EYE_GRID_READ: the caller's tables are older than k_eye_grid)
+    if (GRID == EYE_GRID_READ) pdl_chain();
     {
+        const bool restart = GRID != EYE_GRID_READ && a.restart[b] != 0, fl = GRID != EYE_GRID_READ && a.flip && a.flip[b];
         const float* hp = a.sig + (int64_t)b * 2 * cells;
         const float* off = a.ii + (int64_t)b * (a.gh + 1) * W1;
         const float* lum = a.lum + (int64_t)b * cells;
         const float* col = a.col + (int64_t)b * 2 * cells;
-        for (int32_t q = tid; q < cells; q += EYE_THREADS) {
-            s_hp[q] = hp[q];
-            s_on[q] = hp[cells + q];
-            s_off[q] = off[q];
-            if (sust) {
-                const float l = lum[q];
-                const int32_t y = q / a.gw, x = q - y * a.gw;
-                s_lum[q] = l;
-                s_ii[(y + 1) * W1 + x + 1] = l;
-            }
-            if (a.chromatic) {
-                s_col[q] = col[q];
-                s_col[cells + q] = col[cells + q];
+        for (int32_t q = tid; q < cells; q += T) {
+            if constexpr (GRID == EYE_GRID_READ) {
+                s_hp[q] = hp[q];
+                s_on[q] = hp[cells + q];
+                s_off[q] = off[q];
+                if (sust) {
+                    const float l = lum[q];
+                    const int32_t y = q / a.gw, x = q - y * a.gw;
+                    s_lum[q] = l;
+                    s_ii[(y + 1) * W1 + x + 1] = l;
+                }
+                if (a.chromatic) {
+                    s_col[q] = col[q];
+                    s_col[cells + q] = col[cells + q];
+                }
+            } else {
+                const EyeCell c = eye_cell<GRID == EYE_GRID_OWN4>(a, b, q, (int64_t)b * cells + q, restart, fl);
+                s_hp[q] = c.hp;
+                s_on[q] = c.on;
+                s_off[q] = c.off;
+                if (sust) {
+                    const int32_t y = q / a.gw, x = q - y * a.gw;
+                    s_lum[q] = c.lum;
+                    s_ii[(y + 1) * W1 + x + 1] = c.lum;
+                }
+                if (a.chromatic) {
+                    s_col[q] = c.blue;
+                    s_col[cells + q] = c.green;
+                }
             }
         }
         if (sust) {                                                // a border of zeros
-            for (int32_t t = tid; t <= a.gw; t += EYE_THREADS) s_ii[t] = 0.0f;
-            for (int32_t t = tid; t <= a.gh; t += EYE_THREADS) s_ii[t * W1] = 0.0f;
+            for (int32_t t = tid; t <= a.gw; t += T) s_ii[t] = 0.0f;
+            for (int32_t t = tid; t <= a.gh; t += T) s_ii[t * W1] = 0.0f;
             __syncthreads();
-            for (int32_t t = tid; t <= a.gw; t += EYE_THREADS) running_sum(s_ii + t, a.gh + 1, W1);      // down the rows,
+            for (int32_t t = tid; t <= a.gw; t += T) running_sum(s_ii + t, a.gh + 1, W1);      // down the rows,
             __syncthreads();
-            for (int32_t t = tid; t <= a.gh; t += EYE_THREADS) running_sum(s_ii + t * W1, W1, 1);        // then along them
+            for (int32_t t = tid; t <= a.gh; t += T) running_sum(s_ii + t * W1, W1, 1);        // then along them
         }
     }
-    for (int32_t first = blockIdx.x * run; first < k1; first += EYE_CHUNK) {
-        if (tid < 4) s_kind[tid] = 0;
-        __syncthreads();                                           // (the grids are in place, the last chunk is out)
-        // the neurons' places, sorted by kind: ballots count a warp's, one atomic per kind and warp reserves theirs
-        int32_t kind[EYE_UNROLL], at[EYE_UNROLL], mine = 0;
-#pragma unroll
-        for (int u = 0; u < EYE_UNROLL; u++) {
-            const int32_t c = chan[u] & 15;
-            kind[u] = cell[u] < 0 ? -1 : c < EYE_ON_TRANSIENT ? 0 : c <= EYE_OFF_TRANSIENT ? 1 : c <= EYE_OFF_SUSTAINED ? 2 : 3;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int32_t n = 0;
+    if (!SORT) __syncthreads();                                    // the grids are in place
+    for (int32_t first = blockIdx.x * run; first < k1; first += chunk) {
+        int32_t count = min(chunk, k1 - first), kind[EYE_UNROLL];
+        if (SORT) {
+            if (tid < 4) s_kind[tid] = 0;
+            __syncthreads();                                           // (the grids are in place, the last chunk is out)
+            // the neurons' places, sorted by kind: ballots count a warp's, one atomic per kind and warp reserves theirs
+            int32_t at[EYE_UNROLL], mine = 0;
 #pragma unroll
             for (int u = 0; u < EYE_UNROLL; u++) {
-                const uint32_t m = __ballot_sync(0xffffffffu, kind[u] == i);
-                if (kind[u] == i) at[u] = n + __popc(m & ((1u << lane) - 1u));
-                n += __popc(m);
+                const int32_t c = chan[u] & 15;
+                kind[u] = cell[u] < 0 ? -1 : c < EYE_ON_TRANSIENT ? 0 : c <= EYE_OFF_TRANSIENT ? 1 : c <= EYE_OFF_SUSTAINED ? 2 : 3;
             }
-            if (lane == i) mine = n;
-        }
-        int32_t base = 0;
-        if (lane < 4 && mine) base = atomicAdd(&s_kind[lane], mine);
 #pragma unroll
-        for (int u = 0; u < EYE_UNROLL; u++) {
-            const int32_t from = __shfl_sync(0xffffffffu, base, kind[u] & 3);
-            if (kind[u] >= 0) at[u] += from;
-        }
-        __syncthreads();
-        int32_t count = 0, before[4];
+            for (int i = 0; i < 4; i++) {
+                int32_t n = 0;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            before[i] = count;
-            count += s_kind[i];
-        }
-#pragma unroll
-        for (int u = 0; u < EYE_UNROLL; u++)
-            if (kind[u] >= 0) {
-                const int32_t e = tid + u * EYE_THREADS;
-                const int32_t bf = kind[u] == 0 ? before[0] : kind[u] == 1 ? before[1] : kind[u] == 2 ? before[2] : before[3];
-                s_order[bf + at[u]] = (uint32_t)e | ((uint32_t)chan[u] << 12);
-                s_rate[e] = __int_as_float(cell[u]);               // its cell, until its rate takes the place
+                for (int u = 0; u < EYE_UNROLL; u++) {
+                    const uint32_t m = __ballot_sync(0xffffffffu, kind[u] == i);
+                    if (kind[u] == i) at[u] = n + __popc(m & ((1u << lane) - 1u));
+                    n += __popc(m);
+                }
+                if (lane == i) mine = n;
             }
-        __syncthreads();
+            int32_t base = 0;
+            if (lane < 4 && mine) base = atomicAdd(&s_kind[lane], mine);
+#pragma unroll
+            for (int u = 0; u < EYE_UNROLL; u++) {
+                const int32_t from = __shfl_sync(0xffffffffu, base, kind[u] & 3);
+                if (kind[u] >= 0) at[u] += from;
+            }
+            __syncthreads();
+            int32_t before[4];
+            count = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                before[i] = count;
+                count += s_kind[i];
+            }
+#pragma unroll
+            for (int u = 0; u < EYE_UNROLL; u++)
+                if (kind[u] >= 0) {
+                    const int32_t e = tid + u * T;
+                    const int32_t bf = kind[u] == 0 ? before[0] : kind[u] == 1 ? before[1] : kind[u] == 2 ? before[2] : before[3];
+                    s_order[bf + at[u]] = (uint32_t)e | ((uint32_t)chan[u] << 12);
+                    s_rate[e] = __int_as_float(cell[u]);               // its cell, until its rate takes the place
+                }
+            __syncthreads();
+        } else {
+#pragma unroll
+            for (int u = 0; u < EYE_UNROLL; u++) {                 // (a thread's own entries, in neuron order)
+                const int32_t e = tid + u * T;
+                s_order[e] = (uint32_t)e | ((uint32_t)chan[u] << 12);
+                s_rate[e] = __int_as_float(cell[u]);
+                kind[u] = cell[u];
+            }
+        }
         // (in turn, so that the code of one neuron is not unrolled four times)
 #pragma unroll 1
-        for (int32_t at_e = tid; at_e < count; at_e += EYE_THREADS) {
+        for (int32_t at_e = tid; at_e < count; at_e += T) {
             const uint32_t o = s_order[at_e];
-            const int32_t e = (int32_t)(o & (EYE_CHUNK - 1)), c = (int32_t)((o >> 12) & 15u), q = __float_as_int(s_rate[e]);
+            const int32_t e = (int32_t)(o & 4095u), c = (int32_t)((o >> 12) & 15u), q = __float_as_int(s_rate[e]);
+            if (!SORT && q < 0) continue;
             const int32_t y = q / a.gw, x = q - y * a.gw;
             float r = 0.0f;
             if (c < EYE_ON_TRANSIENT) {
@@ -525,16 +586,16 @@ __global__ void __launch_bounds__(EYE_THREADS) k_eye_neurons(const EyeArgs a, co
             if (!((o >> 16) & 1u)) r = 0.0f;
             s_rate[e] = __fmul_rn(a.max_rate, fminf(fmaxf(__fmul_rn(a.gain_f, r), 0.0f), 1.0f));
         }
-        __syncthreads();
+        if (SORT) __syncthreads();
 #pragma unroll
         for (int u = 0; u < EYE_UNROLL; u++) {
             if (kind[u] < 0) continue;
-            const int32_t e = tid + u * EYE_THREADS;
+            const int32_t e = tid + u * T;
             const float rate = s_rate[e];
             if (a.rates) a.rates[(int64_t)b * a.n_cells + first + e] = rate;
             a.p_ext[(int64_t)b * a.n_ext + slot[u]] = __fmul_rn(rate, a.p_scale);
         }
-        if (first + EYE_CHUNK < k1) fetch(first + EYE_CHUNK);
+        if (first + chunk < k1) fetch(first + chunk);
     }
     if (blockIdx.x == 0 && tid == 0) a.restart[b] = 0;
 }

@@ -782,6 +782,17 @@ extern "C" int64_t fb_eye_state_floats(int32_t batch, int32_t H, int32_t W, int3
     return (int64_t)batch * (8 * gh * gw + (gh + 1) * (gw + 1));
 }
 
+namespace {
+// The neuron kernel of T threads that forms the grids itself (one launch; wide: cells of 4 x 4 aligned pixels) or reads them
+template <int T>
+void (*eye_neurons(bool one, bool wide, bool sort))(const EyeArgs, const EyeSmem, int32_t)
+{
+    if (!one) return sort ? k_eye_neurons<EYE_GRID_READ, true, T> : k_eye_neurons<EYE_GRID_READ, false, T>;
+    if (wide) return sort ? k_eye_neurons<EYE_GRID_OWN4, true, T> : k_eye_neurons<EYE_GRID_OWN4, false, T>;
+    return sort ? k_eye_neurons<EYE_GRID_OWN, true, T> : k_eye_neurons<EYE_GRID_OWN, false, T>;
+}
+}  // namespace
+
 extern "C" int fb_motion_eye(fb_brain* h, const uint8_t* frames, int32_t H, int32_t W, const fb_eye_params* ep,
                              float* state, uint8_t* restart, const uint8_t* flip, int32_t n_cells, const int32_t* gx,
                              const int32_t* gy, const uint8_t* chan, const uint8_t* visible, const int32_t* slot,
@@ -808,25 +819,45 @@ extern "C" int fb_motion_eye(fb_brain* h, const uint8_t* frames, int32_t H, int3
     a.n_cells = n_cells; a.gx = gx; a.gy = gy; a.chan = chan; a.visible = visible; a.slot = slot;
     a.p_ext = h->p_ext; a.n_ext = (int32_t)h->n_ext; a.rates = rates;
     cudaStream_t st = (cudaStream_t)stream;
-    // kernels 1 promises a grid that one block could hold in shared memory (luminance, signals, delay arms,
-    // colours, integral image, contrast); the two-launch form needs the integral image there
+    // kernels 1 promises a grid that one block could hold in shared memory with luminance, signals, delay arms, colours,
+    // integral image, contrast and its tables; k_eye_neurons needs less
     const int64_t grid = (int64_t)gh * gw, ii = (int64_t)(gh + 1) * (gw + 1);
     const bool sust = ep->sustained_gain != 0.0;
     const int64_t block = grid * (8 * sust + 4 * (5 + 2 * a.chromatic)) + ii * 4 * sust + (766 + 256) * 4;
     if (ep->kernels == 1 && block > 227 * 1024)
         return fail(FB_ERR_ARG, "eye grid too large for one block's shared memory");
-    const EyeSmem S(grid, ii, sust, a.chromatic != 0);
-    if (ep->kernels != 2 && S.total * 4 <= EYE_SMEM_MAX && h->B <= 65535) {
+    if (ep->kernels != 2 && EyeSmem(EYE_THREADS, gh * gw, (gh + 1) * (gw + 1), sust, a.chromatic != 0).total * 4 <= EYE_SMEM_MAX && h->B <= 65535) {
         const bool wide = ep->cell == 4 && W % 4 == 0 && ((uintptr_t)frames & 3) == 0;
+        // More instances than SMs: half-sized blocks, two to an SM, where their grids fit twice (us per call, 160 eyes of
+        // 1,000 cells and 1,000 neurons: 14.0 and 16.7)
+        const EyeSmem S2(EYE_THREADS / 2, gh * gw, (gh + 1) * (gw + 1), sust, a.chromatic != 0);
+        const bool half = h->B > h->sm_count && S2.total * 4 <= (EYE_SMEM_MAX - 1024) / 2;
+        const int32_t threads = half ? EYE_THREADS / 2 : EYE_THREADS;
+        const EyeSmem S = half ? S2 : EyeSmem(EYE_THREADS, gh * gw, (gh + 1) * (gw + 1), sust, a.chromatic != 0);
+        // One launch, a block per instance that takes its grid too, saves 1-2 us of launch and a pass over the grids; two
+        // spread an instance over the SMs that are idle otherwise. So one where the work of a block (in cells of
+        // 4 x 4 pixels; a neuron is half of one) times the square of the idle share of the chip is small. us, one launch / two /
+        // one block per instance as a kernel of its own before: 30 x 256 cells, 1,000 neurons 6.7 / 7.7 / 7.5; 30 x 1,000, 1,000
+        // 8.7 / 8.1 / 10.3; 30 x 1,000, 3,287 11.6 / 11.8 / 14.8; 64 x 2,000, 1,000 11.9 / 12.8 / 14.7; 64 x 2,000, 6,000 20.0 / 15.3 / 22.6;
+        // 148 x 1,000, 1,000 8.9 / 12.3 / 10.6. Slower than that kernel: motion channels alone of more instances than SMs
+        // (160 x 1,000 cells, 3,287 neurons 12.9 and 11.2: it held two blocks of 1,024 threads an SM, at 32 registers).
+        const int32_t slots = h->sm_count * (half ? 2 : 1), waves = (h->B + slots - 1) / slots;
+        const double idle = 1.0 - (double)h->B / ((double)slots * waves);
+        const double work = ((double)grid * ep->cell * ep->cell / 16.0 + 0.5 * n_cells) * waves * (half ? 2 : 1);
+        const bool one = work * idle * idle <= 860.0;
+        // blocks per instance: enough to fill the SMs once, at least EYE_THREADS neurons each
+        const int32_t per = one ? 1 : std::max(1, std::min(h->sm_count / h->B, (n_cells + EYE_THREADS - 1) / EYE_THREADS));
+        const int32_t run = std::max(1, (n_cells + per - 1) / per);
+        // sorted by kind where the contrast's FP64 would hold up whole warps for long enough: with 820 neurons a block 11.2 us
+        // unsorted and 12.3 sorted (30 x 1,000 cells, 3,287 neurons), with 1,644 13.0 and 13.1, with 3,000 15.2 and 14.1
+        const bool sort = sust && run > EYE_THREADS + EYE_THREADS / 2;
+        const auto neurons = half ? eye_neurons<EYE_THREADS / 2>(one, wide, sort) : eye_neurons<EYE_THREADS>(one, wide, sort);
         // before the first launch, so that a refusal would leave the filters as they were; to the most any eye
         // needs, so that a concurrent call for a smaller one does not lower it
-        if (S.total * 4 > 48 * 1024) CU(cudaFuncSetAttribute(k_eye_neurons, cudaFuncAttributeMaxDynamicSharedMemorySize, EYE_SMEM_MAX));
-        CU(launch_chain(wide ? k_eye_grid<true> : k_eye_grid<false>, (unsigned)((cells + 255) / 256), 256, 0, st, 1, 1, a));
-        // blocks per instance: enough to fill the SMs once, at least EYE_THREADS neurons each
-        const int32_t per = std::max(1, std::min(h->sm_count / h->B, (n_cells + EYE_THREADS - 1) / EYE_THREADS));
-        const int32_t run = std::max(1, (n_cells + per - 1) / per);
-        CU(launch_chain(k_eye_neurons, dim3((unsigned)per, (unsigned)h->B), EYE_THREADS, (size_t)S.total * 4, st, 1, 1, a, S, run));
-        h->launches += 2;
+        if (S.total * 4 > 48 * 1024) CU(cudaFuncSetAttribute(neurons, cudaFuncAttributeMaxDynamicSharedMemorySize, EYE_SMEM_MAX));
+        if (!one) CU(launch_chain(wide ? k_eye_grid<true> : k_eye_grid<false>, (unsigned)((cells + 255) / 256), 256, 0, st, 1, 1, a));
+        CU(launch_chain(neurons, dim3((unsigned)per, (unsigned)h->B), threads, (size_t)S.total * 4, st, 1, 1, a, S, run));
+        h->launches += one ? 1 : 2;
         return FB_OK;
     }
     int launches = 2;

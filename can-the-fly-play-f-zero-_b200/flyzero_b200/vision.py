@@ -163,7 +163,8 @@ def _p(t):
 class BatchMotionEye:
     """One ``MotionEye`` per instance of ``brain``; ``see`` drives the eye neurons' Poisson input.
     ``kernels``: "fused" runs a grid kernel and a neuron kernel that keeps the instance's grids in
-    shared memory, "split" runs four grid-wide kernels, "auto" the first when it fits."""
+    shared memory (small eyes: the latter alone, forming the grids itself), "split" runs four grid-wide
+    kernels, "auto" the first when it fits."""
 
     def __init__(self, brain, conn, frame_shape, params: MotionParams | None = None, eye_layout: EyeLayout | None = None,
                  kernels: str = "auto"):

@@ -207,7 +207,7 @@ int fb_backprop(const fb_brain* brain, const int32_t* sel, const int32_t* pre_l,
  * (vision.py:34-50): a_hp = float32(1 / tau_hp), a_d = float32(1 / tau_delay), p_scale =
  * float32(dt / 1000); chromatic_gain > 0 computes the blue / green channels, sustained_gain != 0
  * the centre-surround contrast. kernels: 0 = a grid kernel and a neuron kernel that holds the
- * instance's grids in shared memory when they fit (else four grid-wide kernels), 1 = the same
+ * instance's grids in shared memory when they fit (one kernel for small eyes; else four grid-wide ones), 1 = the same
  * (FB_ERR_ARG if they do not fit), 2 = the four grid-wide kernels. */
 typedef struct fb_eye_params {
     int32_t cell, shift, surround, kernels;
