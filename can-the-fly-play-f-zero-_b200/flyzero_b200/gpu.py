@@ -290,11 +290,12 @@ class BatchBrain:
 
     # ---- schedule autotuner -------------------------------------------------------------------
     def schedule_candidates(self):
-        """Schedules worth timing for this engine: (engine, propagation, lanes)."""
+        """Schedules worth timing for this engine: (engine, propagation, lanes). The persistent engine has
+        one: lanes are the step engine's (timed with three, the same kernel won or lost to itself by noise)."""
         info = self.info()
         cands = []
         if info.group > 0 and not info.f64:
-            cands += [("persistent", "push", lanes) for lanes in (8, 16, 32)]
+            cands.append(("persistent", "push", 8))
         cands += [("step", "push", 8), ("step", "push", 32), ("step", "pull", 8)]
         return cands
 
