@@ -107,7 +107,8 @@ class BatchMotor:
         _lib.check(b._L.fb_group_rates(b._h, _p(counts), _p(self.g.idx), _p(self.g.ptr), self.g.n_groups, _p(self.w),
                                        float(a), float(hz), _p(self.rates_dev), _stream(b.device)))
         rates = self.rates
-        if type(self).buttons is not BatchMotor.buttons or self.p.taps:
+        # (a subclass's or an instance's own rule is asked slot by slot)
+        if getattr(self.buttons, "__func__", None) is not BatchMotor.buttons or self.p.taps:
             return [self.buttons(r, k) for k, r in enumerate(rates)]
         return self._all_buttons(rates)
 
