@@ -420,12 +420,12 @@ __global__ void __launch_bounds__(T, EYE_THREADS / T) k_eye_neurons(const EyeArg
     const int32_t cells = a.gh * a.gw;
     float *s_hp = sm + S.hp, *s_on = sm + S.on, *s_off = sm + S.off, *s_lum = sm + S.lum, *s_ii = sm + S.ii;
     float *s_col = sm + S.col, *s_rate = sm + S.rate;
-    uint32_t* s_order = reinterpret_cast<uint32_t*>(sm + S.order); // per sorted place: entry | channel << 12 | visible << 16
+    uint32_t* s_order = reinterpret_cast<uint32_t*>(sm + S.order); // per sorted place: entry | channel << 12 | visible << 16 | y << 17
     int32_t* s_kind = reinterpret_cast<int32_t*>(sm + S.kind);     // neurons of each kind in the chunk
     const bool sust = a.sustained != 0.0;
     const int32_t k1 = min(a.n_cells, (int32_t)(blockIdx.x + 1) * run);
     // a chunk's neurons, loaded ahead (the first one's beside the grids): cell (-1: out of range, or no neuron),
-    // channel and visibility, ext slot
+    // channel, visibility and row (no division by gw later: 5 % of the instructions), ext slot
     int32_t cell[EYE_UNROLL], chan[EYE_UNROLL], slot[EYE_UNROLL];
     auto fetch = [&](int32_t first) {
 #pragma unroll
@@ -435,9 +435,11 @@ __global__ void __launch_bounds__(T, EYE_THREADS / T) k_eye_neurons(const EyeArg
             chan[u] = slot[u] = 0;
             if (k >= k1) continue;
             const int32_t x = __ldg(a.gx + k), y = __ldg(a.gy + k), c = __ldg(a.chan + k);
+            const int32_t seen = __ldg(a.visible + k) != 0;
             slot[u] = __ldg(a.slot + k);
-            chan[u] = c | ((int32_t)(__ldg(a.visible + k) != 0) << 4);
-            if (x >= 0 && x < a.gw && y >= 0 && y < a.gh && c < EYE_CHANNELS && slot[u] >= 0 && slot[u] < a.n_ext) cell[u] = y * a.gw + x;
+            const bool in = x >= 0 && x < a.gw && y >= 0 && y < a.gh && c < EYE_CHANNELS && slot[u] >= 0 && slot[u] < a.n_ext;
+            if (in) cell[u] = y * a.gw + x;
+            chan[u] = (c & 15) | (seen << 4) | ((y & 1023) << 5);
         }
     };
     if (GRID != EYE_GRID_READ) pdl_chain();
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(T, EYE_THREADS / T) k_eye_neurons(const EyeArg
             const uint32_t o = s_order[at_e];
             const int32_t e = (int32_t)(o & 4095u), c = (int32_t)((o >> 12) & 15u), q = __float_as_int(s_rate[e]);
             if (!SORT && q < 0) continue;
-            const int32_t y = q / a.gw, x = q - y * a.gw;
+            const int32_t y = (int32_t)(o >> 17), x = q - y * a.gw;
             float r = 0.0f;
             if (c < EYE_ON_TRANSIENT) {
                 const int32_t dir = c & 3, sh = a.shift;
