@@ -186,6 +186,7 @@ struct PersistCnt {
     int32_t n_spk[2];                        // spikes buffered (epoch parity)
     int32_t entries[2];                      // entries scattered in the last epoch (epoch parity)
     int32_t stop;
+    int32_t list_at, count_at;               // where the epoch's first step lies in the rings of lists and of their lengths
     int32_t cursor[MAX_EPOCH], base[MAX_EPOCH];  // a listing batch's items per step, and where they start in the lists
 };
 static_assert(sizeof(PersistCnt) <= 512, "counters fit their block");
@@ -288,10 +289,22 @@ __device__ __forceinline__ void list_one(const PersistParams& P, int32_t k, int3
     }
 }
 
-// Its work items at `base`, .. of its step's list
-__device__ __forceinline__ void write_items(const PersistParams& P, int64_t t, int32_t base, int64_t r0, int64_t r1, int32_t b)
+// A place in a ring of m at most m - 1 before or behind it
+__device__ __forceinline__ int32_t wrap(int32_t at, int32_t m) { return at < 0 ? at + m : at >= m ? at - m : at; }
+// The list of the step `ds` steps after (before: < 0) the epoch's first and its length. By the tick, list_of and count_of
+// take a 64-bit remainder each, and an epoch's chain of listing, pushing and advancing had six of them
+__device__ __forceinline__ int2* list_from(const PersistParams& P, int32_t ds)
 {
-    int2* list = list_of(P.N, P.S, t, P.q);
+    return P.S.items + ((int64_t)wrap(smem_at<PersistCnt>(P.lay.misc)->list_at + ds, P.N.R) * P.S.n_groups + P.q) * P.S.cap_c;
+}
+__device__ __forceinline__ int32_t* count_from(const PersistParams& P, int32_t ds)
+{
+    return P.S.item_count + wrap(smem_at<PersistCnt>(P.lay.misc)->count_at + ds, P.N.R_pl) * P.S.n_groups + P.q;
+}
+
+// Its work items at `base`, .. of its step's list
+__device__ __forceinline__ void write_items(const PersistParams& P, int2* list, int32_t base, int64_t r0, int64_t r1, int32_t b)
+{
     for (int64_t r = r0; r < r1; r += CHUNK, base++) {
         if (base < P.S.cap_c) list[base] = make_int2((int32_t)r, (b << CHUNK_BITS) | (int32_t)min((int64_t)CHUNK, r1 - r));
         else atomicExch(P.S.err, 1);
@@ -308,7 +321,7 @@ __device__ __noinline__ void list_overflow(const PersistParams& P, int32_t k, in
     list_one<PLASTIC, RECORD>(P, k, s, r0, r1, b);
     const int64_t t = P.A.t0 + s;
     const int nch = row_items(r0, r1);
-    if (nch) write_items(P, t, atomicAdd(count_of(P.N, P.S, t, P.q), nch), r0, r1, b);
+    if (nch) write_items(P, list_of(P.N, P.S, t, P.q), atomicAdd(count_of(P.N, P.S, t, P.q), nch), r0, r1, b);
 }
 
 // The spikes of local pair k (bit 4 s: at step s of the epoch whose first step is s0) into the buffer of
@@ -329,9 +342,9 @@ __device__ __forceinline__ void record_spikes(const PersistParams& P, int par, i
 // The buffered spikes (parity par) of the epoch whose first step is s0 (kc steps): counts, plastic rows,
 // records, work items. A batch of `stride` spikes (one per thread) reserves its items with one atomic
 // per step. Threads tid0 = 0..stride-1: the listing warps, or (`all`) the whole block; the counters of
-// the parity are zero again afterwards.
+// the parity are zero again afterwards. `back`: steps from that epoch to the present one.
 template <bool PLASTIC, bool RECORD>
-__device__ __noinline__ void list_epoch(const PersistParams& P, int par, int32_t s0, int32_t kc, bool all)
+__device__ __noinline__ void list_epoch(const PersistParams& P, int par, int32_t s0, int32_t kc, int32_t back, bool all)
 {
     PersistCnt* C = smem_at<PersistCnt>(P.lay.misc);
     const uint32_t* spk = smem_at<uint32_t>(P.lay.spk) + par * SPK_BUF;
@@ -355,10 +368,10 @@ __device__ __noinline__ void list_epoch(const PersistParams& P, int par, int32_t
         if (tid0 < kc) {
             const int32_t n = C->cursor[tid0];
             C->cursor[tid0] = 0;
-            C->base[tid0] = n ? atomicAdd(count_of(P.N, P.S, P.A.t0 + s0 + tid0, P.q), n) : 0;
+            C->base[tid0] = n ? atomicAdd(count_from(P, tid0 - back), n) : 0;
         }
         sync();
-        if (r1 > r0) write_items(P, P.A.t0 + s0 + ds, C->base[ds] + at, r0, r1, b);
+        if (r1 > r0) write_items(P, list_from(P, ds - back), C->base[ds] + at, r0, r1, b);
     }
     sync();
     if (tid0 == 0) C->n_spk[par] = 0;
@@ -437,9 +450,10 @@ __device__ __noinline__ void draw_kicks(const PersistParams& P, int32_t s0, int 
 // step and CTA. ms with 5 and 7 warps, by entries: 35 thousand (16 whole brains, 30 % driven at 100 Hz) 9.9 and
 // 7.8; 15 thousand (16 x 20,000, 300 entries a row, all at 60 Hz) 2.35 and 2.18; 10 thousand (16 x 50,000, all
 // at 400 Hz) 2.29 and 2.29; 5 thousand (half of them) 1.38 and 1.60. Sums are whole numbers: who pushes
-// an item does not matter. `next`: the coming epoch's parity.
+// an item does not matter. `ahead`: steps from the present epoch's first tick to a0; `slot0`: the accumulator slot of
+// that tick; `next`: the coming epoch's parity.
 template <typename AccT>
-__device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int64_t a1, int w, int n_w, int next)
+__device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int64_t a1, int ahead, int slot0, int w, int n_w, int next)
 {
     constexpr unsigned FULL = 0xffffffffu;
     const DevNet& N = P.N;
@@ -450,9 +464,11 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
     // this CTA's share of each list, flattened
     int32_t from = 0, len_k = 0;
     if (lane < nl && a0 + lane >= N.n_delay) {
-        const int64_t total = list_length(N, S, a0 + lane - N.n_delay, P.q);
-        from = (int32_t)(total * blockIdx.x / gridDim.x);
-        len_k = (int32_t)(total * (blockIdx.x + 1) / gridDim.x) - from;
+        // total * block / blocks in 32 bits: by its quotient and remainder
+        const uint32_t total = (uint32_t)min((int64_t)max(__ldcg(count_from(P, ahead + lane - N.n_delay)), 0), S.cap_c);
+        const uint32_t n_c = gridDim.x, c = blockIdx.x, each = total / n_c, rest = total - each * n_c;
+        from = (int32_t)(each * c + rest * c / n_c);
+        len_k = (int32_t)(each * (c + 1) + rest * (c + 1) / n_c) - from;
     }
     int32_t first[MAX_EPOCH], off[MAX_EPOCH + 1];
     off[0] = 0;
@@ -461,12 +477,14 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
         first[k] = __shfl_sync(FULL, from, k);
         off[k + 1] = off[k] + __shfl_sync(FULL, len_k, k);
     }
-    const int64_t M = off[MAX_EPOCH], np = N.n_pad, slot_stride = (int64_t)N.B * np;
+    const uint32_t M = (uint32_t)off[MAX_EPOCH];                // (at most six lists of 2^31 by 148: 16 M fits)
+    const int64_t np = N.n_pad, slot_stride = (int64_t)N.B * np;
     AccT* acc0 = reinterpret_cast<AccT*>(S.acc) + (int64_t)P.b0 * np;
-    const int32_t slot0 = (int32_t)pos_mod(a0, S.n_slots), list0 = (int32_t)pos_mod(a0 - N.n_delay, N.R);
-    const int32_t j1 = (int32_t)(M * (w + 1) / n_w);
+    const int32_t list0 = wrap(smem_at<PersistCnt>(P.lay.misc)->list_at + ahead - N.n_delay, N.R);
+    slot0 = wrap(slot0 + ahead, S.n_slots);
+    const int32_t j1 = (int32_t)(M * (uint32_t)(w + 1) / (uint32_t)n_w);
     int32_t mine = 0;
-    for (int32_t j0 = (int32_t)(M * w / n_w); j0 < j1; j0 += 32) {
+    for (int32_t j0 = (int32_t)(M * (uint32_t)w / (uint32_t)n_w); j0 < j1; j0 += 32) {
         int32_t start = 0, len = 0;
         int64_t to = 0;                                         // offset of the item's row of accumulators
         if (j0 + lane < j1) {
@@ -499,8 +517,10 @@ __device__ __noinline__ void push_epoch(const PersistParams& P, int64_t a0, int6
             }
         }
     }
-    mine = __reduce_add_sync(FULL, mine);
-    if (lane == 0 && mine) atomicAdd(&smem_at<PersistCnt>(P.lay.misc)->entries[next], mine);
+    if (M > BUSY_ENTRIES / CHUNK) {                             // (fewer items cannot hold that many entries)
+        mine = __reduce_add_sync(FULL, mine);
+        if (lane == 0 && mine) atomicAdd(&smem_at<PersistCnt>(P.lay.misc)->entries[next], mine);
+    }
 }
 
 // The pair-by-pair advance of up to 8 quads through the kc steps of the epoch whose first is s0, four
@@ -722,6 +742,10 @@ __device__ __noinline__ void load_state(const PersistParams& P, int32_t cnt)
         smem_at<uint32_t>(P.lay.hash)[MAX_EPOCH * 64 + tid] = (uint32_t)((int64_t)(b0 + tid) * n + lo - (int64_t)tid * np);
     }
     __syncthreads();
+    if (tid == 0) {
+        C->list_at = (int32_t)pos_mod(P.A.t0, N.R);
+        C->count_at = (int32_t)pos_mod(P.A.t0, N.R_pl);
+    }
     prepare_epoch<RASTER>(P, 0, min(P.A.epoch, P.A.steps), 0, tid, PT);
     const int32_t e0 = P.A.ext_off[blockIdx.x], e1 = P.A.ext_off[blockIdx.x + 1];
     int2* s_in = smem_at<int2>(P.lay.inputs);
@@ -786,7 +810,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
     {
         const int64_t a1 = min(A.t0 + K, A.t0 + A.steps + 1);
         if (A.pushed_until < a1) {
-            push_epoch<AccT>(P, A.pushed_until, a1, tid >> 5, PT / 32, 0);
+            push_epoch<AccT>(P, A.pushed_until, a1, (int)(A.pushed_until - A.t0), slot0, tid >> 5, PT / 32, 0);
             __syncthreads();
             bar_target += gridDim.x;
             if (tid == 0) {
@@ -805,10 +829,10 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
         if (tid == PT - 1 && A.trace) c_begin = clock64();
         if (is_l) {
             const int32_t kc = min(K, A.steps - ep0);
-            if (A.list_late && ep0 > 0) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, K, false);
+            if (A.list_late && ep0 > 0) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, K, K, false);
             // the lists whose items arrive in this epoch were pushed before it: their lengths are zero when the
             // slots serve again, K steps after the ticks of this epoch
-            if (blockIdx.x == 0 && tid < kc) *count_of(P.N, P.S, A.t0 + ep0 + tid - P.N.n_delay, P.q) = 0;
+            if (blockIdx.x == 0 && tid < kc) *count_from(P, tid - P.N.n_delay) = 0;
             if (ep0 + kc < A.steps) prepare_epoch<RASTER>(P, ep0 + kc, min(K, A.steps - ep0 - kc), par ^ 1, tid, LIST_THREADS);
             if (tid == 0) {
                 C->tile[par ^ 1] = 0;
@@ -820,7 +844,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
             const int64_t end = A.t0 + A.steps + 1, T = A.t0 + ep0;
             const int64_t pa0 = max(A.pushed_until, min(T + K, end)), pa1 = min(T + 2 * K, end);
             if (tid == LIST_THREADS) stamp(A, ep0, 7);
-            if (pa0 < pa1) push_epoch<AccT>(P, pa0, pa1, (tid - LIST_THREADS) >> 5, n_w, par ^ 1);
+            if (pa0 < pa1) push_epoch<AccT>(P, pa0, pa1, (int)(pa0 - T), slot0, (tid - LIST_THREADS) >> 5, n_w, par ^ 1);
             if (tid == LIST_THREADS) stamp(A, ep0, 10);
         }
         // ---- advance: the special quads first (8 of them per turn), then the tiles ---------------------
@@ -853,16 +877,18 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
         if (ring0 >= P.N.R_pl) ring0 -= P.N.R_pl;
         if (!A.list_late) {
             __syncthreads();                                    // every spike of the epoch is buffered
-            list_epoch<PLASTIC, RECORD>(P, par, ep0, kc, true);
+            list_epoch<PLASTIC, RECORD>(P, par, ep0, kc, 0, true);
         }
         if (ep0 + K < A.steps) {                                // another epoch follows
             __syncthreads();                                    // this epoch's work of the CTA is done
             long long c0 = 0;
             if (tid == 0) {
                 c0 = clock64();
-                C->entries[par] = 0;                            // (the coming epoch adds to it)
                 grid_arrive(A);
                 stamp(A, ep0 + K - 1, 5);
+                C->entries[par] = 0;                            // (the coming epoch adds to it)
+                C->list_at = wrap(C->list_at + K, P.N.R);
+                C->count_at = wrap(C->count_at + K, P.N.R_pl);
             }
             draw_kicks<RASTER, KB>(P, ep0 + K, par ^ 1);
             bar_target += gridDim.x;
@@ -877,7 +903,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist(const __grid_constant__ Persi
     }
     // the last epoch's spikes are listed before the launch ends (the next launch scatters them)
     __syncthreads();
-    if (!stop && A.list_late) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, A.steps - (ep0 - K), true);
+    if (!stop && A.list_late) list_epoch<PLASTIC, RECORD>(P, par ^ 1, ep0 - K, A.steps - (ep0 - K), 0, true);
     store_state(P, cnt);
 }
 
