@@ -37,9 +37,13 @@ METRIC = "sim neuron-steps/s (138k LIF, B=64 batched vs B=1 plain) at matched ra
 UNIT = "neuron-steps/s"
 DT = 0.1
 PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
+# what a step moves when nothing stays on chip
 BYTES_PER_NEURON_STEP = 26        # v r/w 8 + g r/w 8 + ref r/w 2 + accumulator read+clear 8
 BYTES_PER_SPIKE = 16              # row pointers 8 + count r/w 8
 BYTES_PER_EDGE = 14               # column 4 + count 2 + accumulator read-modify-write 8
+# what a frame cannot do without: every neuron's state in and out once and its count, every entry once
+BYTES_PER_NEURON_FRAME = 22       # v r/w 8 + g r/w 8 + ref r/w 2 + count 4
+BYTES_PER_ENTRY_FRAME = 6         # column 4 + count 2
 
 
 def parse():
@@ -308,20 +312,15 @@ def spike_bytes(counts_list, rowlen_dev):
 
 
 def dram_traffic_record():
-    """DRAM bytes (read + write) of one persistent-kernel launch of this workload, read from the
-    committed ncu summary of that kernel (its 'traffic per launch' line names the commit and the
-    command it was measured at); None if the record is missing."""
-    import re
-
-    path = os.path.join(ROOT, "profiles", "k_persist_b64_138k.md")
+    """DRAM bytes (read + write) of one persistent-kernel launch of this workload as ncu counted them, and
+    where that is recorded (file and commit); None if the record is missing."""
+    name = "profiles/k_persist_b64_138k.json"
     try:
-        text = open(path).read()
+        with open(os.path.join(ROOT, name)) as f:
+            rec = json.load(f)
     except OSError:
         return None, None
-    m = re.search(r"traffic-per-launch-bytes:\s*([0-9_]+)\s+\(commit ([0-9a-f]+)", text)
-    if not m:
-        return None, None
-    return int(m.group(1).replace("_", "")), f"profiles/k_persist_b64_138k.md, commit {m.group(2)}"
+    return int(rec["dram_bytes_per_launch"]), f"{name}, commit {rec['commit']}"
 
 
 class Episodes:
@@ -463,11 +462,12 @@ def run_ours(args, world, rank, local):
     neuron_steps = active * n
     value, max_ms = replica_value(neuron_steps, elapsed_ms, world)
     spk, edges = spike_bytes(counts[args.warmup:], rowlen)
-    alg_bytes = BYTES_PER_NEURON_STEP * neuron_steps + BYTES_PER_SPIKE * spk + BYTES_PER_EDGE * edges
+    step_bytes = BYTES_PER_NEURON_STEP * neuron_steps + BYTES_PER_SPIKE * spk + BYTES_PER_EDGE * edges
     info = gb.info()
     peak, peak_kind = peaks()
     n_kern = max(1, loop.run_launches - l_run0)   # the runs' launches: one per instance group per frame
-    achieved = (alg_bytes / n_kern) / (run_ms / 1000.0 / n_kern) / 1e9
+    frame_bytes = args.steps * (BYTES_PER_NEURON_FRAME * B * n + BYTES_PER_ENTRY_FRAME * int(conn.nnz))
+    achieved = frame_bytes / (run_ms / 1000.0) / 1e9
     traffic, traffic_src = dram_traffic_record()
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -495,8 +495,12 @@ def run_ours(args, world, rank, local):
                      "kernel_ms_per_launch": run_ms / n_kern, "kernel_launches": n_kern,
                      "kernel_timing": "CUDA events on the launching stream around each frame's run (its "
                                       "persistent launches) inside the timed loop",
-                     "model": "26 B per instance-neuron-step + 16 B per spike + 14 B per edge pushed, per launch of the "
-                              "persistent kernel (one per instance group per frame)"},
+                     "model": "22 B per instance-neuron and 6 B per connectome entry, once a frame: state in and out, "
+                              "counts, connectome; what a step moves beside them stays in shared memory and L2, so that "
+                              "reductions and barriers bound the kernel, not HBM",
+                     "on_chip_gbs": step_bytes / (run_ms / 1000.0) / 1e9,
+                     "on_chip_model": "26 B per instance-neuron-step + 16 B per spike + 14 B per edge pushed",
+                     "reductions_per_s": edges / (run_ms / 1000.0)},
         "gpu_launches": launches,
         "clocks": clk,
     }
@@ -1011,6 +1015,11 @@ def run_instruct(args, world, rank, local):
             "mean_rate_error_hz_last_frame": err, "clocks": clk}), flush=True)
 
 
+# the phases that the persistent engine stamps itself (an epoch's span is divided evenly between its steps, so the
+# others are nil)
+TRACED = ("step", "neuron_loop", "neuron_loop_max_over_ctas", "listing", "push_per_epoch", "grid_barrier_wait")
+
+
 def run_trace(args, world, rank, local):
     """Phase trace of the persistent engine on the headline workload (a diagnostic): after
     --warmup frames, one frame with fb_set_trace on, then untraced frames until a second has passed;
@@ -1058,7 +1067,7 @@ def run_trace(args, world, rank, local):
             "config": {"workload": f"headline workload, {args.batch} instances x 138,639 neurons, one traced frame of "
                                    f"{fs} steps; the last instance group's launch", "epoch_steps": K,
                        "ctas": int(T.shape[1]), "clock_mhz_used": mhz},
-            "phases_us": {k: round(v, 3) for k, v in ph.items()}, "clocks": clk}), flush=True)
+            "phases_us": {k: round(ph[k], 3) for k in TRACED}, "clocks": clk}), flush=True)
 
 
 def main():

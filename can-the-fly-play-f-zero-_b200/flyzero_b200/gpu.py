@@ -28,7 +28,9 @@ TRACE_SLOTS = 11
 
 def phase_summary(T, epoch: int, sm_mhz: float) -> dict:
     """Medians over steps and CTAs (microseconds at ``sm_mhz``) of a phase trace from
-    ``BatchBrain.phase_trace``."""
+    ``BatchBrain.phase_trace``. The persistent engine advances the steps of an epoch together and stamps each with an
+    even share of its span: ``step``, ``neuron_loop`` and its maximum are averages over an epoch, the phases
+    between stamps 0, 4, 1 and 2 are nil."""
     T = np.asarray(T, np.float64) / float(sm_mhz)
     K = int(epoch)
     med = lambda a: float(np.median(a)) if a.size else float("nan")
