@@ -21,6 +21,11 @@ __device__ __forceinline__ void pdl_chain()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The two halves apart, for a kernel whose successor is better set up late: a successor's blocks settle on the SMs
+// that have room when they are let go, all of them on a few where this kernel fills the others.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // The same for a kernel whose successor reads, before its own wait, what was in memory before this kernel
 // began: the successor starts when all that has completed.
 __device__ __forceinline__ void pdl_chain_behind()

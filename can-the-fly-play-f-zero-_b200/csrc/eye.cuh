@@ -229,10 +229,12 @@ __global__ void k_eye_delay(const EyeArgs a)
 // ---- the same eye in two launches or one (the default) ---------------------------------------------------
 // The grid of every instance by one thread per cell, then the neurons of an instance by several blocks.
 // One block per instance for all of it (its grid in shared memory) kept 64 instances on 64 of the 148 SMs and
-// waited through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16.5,
-// 22.0 together as a dependent chain whose second kernel reads its tables beside the first (23.3 without
-// that, 26.6 as ordinary launches). Small eyes, and as many as there are SMs, lose more by the second launch
-// than they gain: they take one block per instance again (fb_motion_eye says where the line lies).
+// waited through its phases one after the other: 38.5 us for 64 frames of 224 x 256; these two take 7.4 and 16,
+// 20.8 together as a dependent chain whose second kernel reads its tables beside the first. The neuron kernel lets
+// the next call's grid kernel go when its blocks are done: let go at once, all the grid's blocks settled on the few SMs
+// that its own blocks had left free (62 eyes of 19 x 19 cells of 8 x 8 pixels: 19.4 us a call, now 10.5). Small
+// eyes, and as many as there are SMs, lose more by the second launch than they gain: they take one
+// block per instance again (fb_motion_eye says where the line lies).
 
 // x / 3 and x / 255 rounded to nearest for the values a pixel can take (R + G + B and its third, a byte): one
 // Newton correction of the quotient by its exact remainder (Markstein 1990). Checked against the
@@ -444,7 +446,7 @@ __global__ void __launch_bounds__(T, EYE_THREADS / T) k_eye_neurons(const EyeArg
     };
     if (GRID != EYE_GRID_READ) pdl_chain();
     fetch(blockIdx.x * run);                                       // (EYE_GRID_READ: the caller's tables are older than k_eye_grid)
-    if (GRID == EYE_GRID_READ) pdl_chain();
+    if (GRID == EYE_GRID_READ) pdl_wait();
     {
         const bool restart = GRID != EYE_GRID_READ && a.restart[b] != 0, fl = GRID != EYE_GRID_READ && a.flip && a.flip[b];
         const float* hp = a.sig + (int64_t)b * 2 * cells;
@@ -599,6 +601,7 @@ __global__ void __launch_bounds__(T, EYE_THREADS / T) k_eye_neurons(const EyeArg
         }
         if (first + chunk < k1) fetch(first + chunk);
     }
+    if (GRID == EYE_GRID_READ) pdl_launch();
     if (blockIdx.x == 0 && tid == 0) a.restart[b] = 0;
 }
 

@@ -834,23 +834,22 @@ extern "C" int fb_motion_eye(fb_brain* h, const uint8_t* frames, int32_t H, int3
         const bool half = h->B > h->sm_count && S2.total * 4 <= (EYE_SMEM_MAX - 1024) / 2;
         const int32_t threads = half ? EYE_THREADS / 2 : EYE_THREADS;
         const EyeSmem S = half ? S2 : EyeSmem(EYE_THREADS, gh * gw, (gh + 1) * (gw + 1), sust, a.chromatic != 0);
-        // One launch, a block per instance that takes its grid too, saves 1-2 us of launch and a pass over the grids; two
-        // spread an instance over the SMs that are idle otherwise. So one where the work of a block (in cells of
-        // 4 x 4 pixels; a neuron is half of one) times the square of the idle share of the chip is small. us, one launch / two /
-        // one block per instance as a kernel of its own before: 30 x 256 cells, 1,000 neurons 6.7 / 7.7 / 7.5; 30 x 1,000, 1,000
-        // 8.7 / 8.1 / 10.3; 30 x 1,000, 3,287 11.6 / 11.8 / 14.8; 64 x 2,000, 1,000 11.9 / 12.8 / 14.7; 64 x 2,000, 6,000 20.0 / 15.3 / 22.6;
-        // 148 x 1,000, 1,000 8.9 / 12.3 / 10.6. Slower than that kernel: motion channels alone of more instances than SMs
-        // (160 x 1,000 cells, 3,287 neurons 12.9 and 11.2: it held two blocks of 1,024 threads an SM, at 32 registers).
+        // One launch, a block per instance that takes its grid too, saves a launch and a pass over the grids; two spread
+        // an instance over the SMs that are idle otherwise. So one where the work of a block (in cells of 4 x 4 pixels; a
+        // neuron is half of one) times the idle share of the chip is small. us, one launch / two / one block per instance
+        // in a kernel of its own before: 30 x 256 cells, 1,000 neurons 6.3 / 6.8 / 7.5; 30 x 1,000, 1,000 8.3 / 7.1 / 10.2;
+        // 64 x 1,000, 300 7.7 / 8.0 / 9.8; 64 x 2,000, 1,000 11.5 / 9.9 / 14.7; 148 x 1,000, 1,000 8.4 / 9.8 / 10.6;
+        // 148 x 3,584, 12,246 34.2 / 36.8 / 42.1; 160 x 1,000, 1,000 13.7 / 12.2 / 15.3.
         const int32_t slots = h->sm_count * (half ? 2 : 1), waves = (h->B + slots - 1) / slots;
         const double idle = 1.0 - (double)h->B / ((double)slots * waves);
         const double work = ((double)grid * ep->cell * ep->cell / 16.0 + 0.5 * n_cells) * waves * (half ? 2 : 1);
-        const bool one = work * idle * idle <= 860.0;
+        const bool one = work * idle <= 700.0;
         // blocks per instance: enough to fill the SMs once, at least EYE_THREADS neurons each
         const int32_t per = one ? 1 : std::max(1, std::min(h->sm_count / h->B, (n_cells + EYE_THREADS - 1) / EYE_THREADS));
         const int32_t run = std::max(1, (n_cells + per - 1) / per);
-        // sorted by kind where the contrast's FP64 would hold up whole warps for long enough: with 820 neurons a block 11.2 us
-        // unsorted and 12.3 sorted (30 x 1,000 cells, 3,287 neurons), with 1,644 13.0 and 13.1, with 3,000 15.2 and 14.1
-        const bool sort = sust && run > EYE_THREADS + EYE_THREADS / 2;
+        // sorted by kind where the contrast's FP64 would hold up whole warps for long enough: with 711 neurons a block 10.5 us
+        // unsorted and 11.7 sorted (3 x 1,210 cells), with 1,030 14.7 and 15.1, with 1,272 11.0 and 10.1, with 3,780 16.3 and 13.9
+        const bool sort = sust && run > EYE_THREADS;
         const auto neurons = half ? eye_neurons<EYE_THREADS / 2>(one, wide, sort) : eye_neurons<EYE_THREADS>(one, wide, sort);
         // before the first launch, so that a refusal would leave the filters as they were; to the most any eye
         // needs, so that a concurrent call for a smaller one does not lower it
