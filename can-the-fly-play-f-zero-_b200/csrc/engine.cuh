@@ -142,30 +142,42 @@ __device__ __forceinline__ int2 make_item(const DevNet& N, int32_t i, int32_t b,
     return make_int2((int32_t)k0, (b << CHUNK_BITS) | (int32_t)min((int64_t)CHUNK, r1 - k0));
 }
 
-// Append `nch` work items (this lane's spike: chunks 0..nch-1 of row i) of instance b, the same for the whole
-// warp, to its group's list; one atomic per warp (the ballot/shuffle compaction).
+// Append `nch` work items (this lane's spike: chunks 0..nch-1 of row i of instance b) to the list of
+// the lane's group; one atomic per warp and list (the ballot/shuffle compaction). The step engine's blocks hold
+// one instance, so one list; written without the search for others its step was slower (100 steps of 16 x 16,384 in
+// FP64: 756 us and 729).
 __device__ __forceinline__ void warp_append(const DevNet& N, const DevState& S, int64_t t, int nch, int32_t i,
                                             int32_t b)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    if (!__any_sync(FULL, nch > 0)) return;
-    int incl = nch;
+    unsigned todo = __ballot_sync(FULL, nch > 0);
+    if (!todo) return;
+    const int32_t key = nch > 0 ? b / S.group : -1;
+    while (todo) {
+        const int leader = __ffs(todo) - 1;
+        const int32_t kk = __shfl_sync(FULL, key, leader);
+        const bool mine = nch > 0 && key == kk;
+        int incl = mine ? nch : 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += y;
-    }
-    const int32_t q = b / S.group;
-    int base = 0;
-    if (lane == 31) base = atomicAdd(count_of(N, S, t, q), incl);
-    base = __shfl_sync(FULL, base, 31);
-    int2* list = list_of(N, S, t, q);
-    const int64_t start = (int64_t)base + incl - nch;
-    for (int ch = 0; ch < nch; ch++) {
-        const int64_t p = start + ch;
-        if (p < S.cap_c) list[p] = make_item(N, i, b, ch);
-        else atomicExch(S.err, 1);
+        for (int o = 1; o < 32; o <<= 1) {
+            int y = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int total = __shfl_sync(FULL, incl, 31);
+        int base = 0;
+        if (lane == 31) base = atomicAdd(count_of(N, S, t, kk), total);
+        base = __shfl_sync(FULL, base, 31);
+        if (mine) {
+            int2* list = list_of(N, S, t, kk);
+            const int64_t start = (int64_t)base + incl - nch;
+            for (int ch = 0; ch < nch; ch++) {
+                const int64_t p = start + ch;
+                if (p < S.cap_c) list[p] = make_item(N, i, b, ch);
+                else atomicExch(S.err, 1);
+            }
+        }
+        todo &= ~__ballot_sync(FULL, mine);
     }
 }
 
@@ -408,8 +420,8 @@ __device__ __forceinline__ void push_lists(const DevNet& N, const DevState& S, i
 // slot is cleared.
 // Small networks are bound by a launch's chain of dependent loads (list length, item, edges;
 // accumulator, state, kick): 16 x 16,384 FP64 took 14.6 us a step as two ordinary launches and takes 7.0,
-// 4 x 1,000 11.7 and 4.0. Large ones are bound by the state's traffic in L2: 16 x 138,639 FP64 30.7
-// and 22.8, 64 x 138,639 FP32 123 and 94.
+// 4 x 1,000 11.7 and 4.0. Large ones are bound by the state's traffic in L2: 16 x 138,639 FP64 30.7 as two
+// launches and 22.8, 64 x 138,639 FP32 123 and 94 (one launch, but a tile a block: 28.5 and 127).
 // ---------------------------------------------------------------------------------------------
 struct StepGrid {
     int32_t n_push, per;       // pushing blocks; updating blocks per instance
