@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(const uint16_t* __restri
 // and B (BN rows) as two 2-D TMA loads (64 bf16 = 128 bytes of K per row, 128-byte swizzle, zeros
 // outside the matrices) into a ring of TMA_STAGES shared-memory stages; one thread issues the
 // tensor-core MMAs from swizzled K-major descriptors as each stage lands and releases the stage with
-// tcgen05.commit; all four warps then read the accumulator from TMEM for the epilogue. No cluster
+// tcgen05.commit; all eight warps then read the accumulator from TMEM for the epilogue. No cluster
 // multicast anywhere. Every wait is bounded; after a timeout no result is written.
 //
 // Split K (gridDim.z = S > 1, launched as clusters of 1 x 1 x S blocks): block z of a cluster
@@ -384,8 +384,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(const uint16_t* __restri
 // partial to its own shared memory (the drained stage ring), and after a cluster barrier each block
 // sums its 1/S share of the tile's rows over the S partials in the order z = 0 .. S-1 through
 // distributed shared memory (ld.shared::cluster, 16 bytes a thread along a row: 512 x 1280 x 4096 in
-// 16.8 us, element by element 24.8, down the columns 41), then applies the epilogue. The sum order is fixed, so a result depends on S and never on
-// scheduling. A second cluster barrier keeps every block's shared memory alive until all reads end.
+// 16.8 us, element by element 24.8, down the columns 41), then applies the epilogue. The sum order is
+// fixed, so a result depends on S and never on scheduling. A second cluster barrier keeps every block's
+// shared memory alive until all reads end.
 // ---------------------------------------------------------------------------------------------
 constexpr int TMA_STAGES = 4;
 constexpr int TMA_THREADS = 256;             // two warps per 32 TMEM lanes: each takes half of a tile's columns (the

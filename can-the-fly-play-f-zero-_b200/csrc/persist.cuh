@@ -21,8 +21,8 @@
 // The listing and pushing warps take tiles too when they are done. One grid barrier ends an epoch;
 // between arriving at it and waiting for it a CTA draws the next epoch's Poisson kicks.
 //
-// What bounds an epoch (16 instances of 138,639 neurons, K = 6: 27 us or 4.5 us per step, against 7.0 for
-// a step-by-step kernel): the advance reads 27 MB of accumulators from L2 and the pushes reduce 1.4 M
+// What bounds an epoch (16 instances of 138,639 neurons, K = 6: 27 us or 4.5 us per step, against 8.4 in the
+// step-by-step kernel before): the advance reads 27 MB of accumulators from L2 and the pushes reduce 1.4 M
 // entries into them, each about half of the 22 us they take together; the barrier takes 3-4 us.
 // Advancing an epoch at a time takes the state's shared-memory traffic (22 B per pair and step) and
 // three CTA-level barriers out of every step. 512 threads: with 128 registers each nothing of the
